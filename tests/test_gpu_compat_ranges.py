@@ -1,0 +1,44 @@
+"""PM_MODE_ZHOU_COMPAT bit for bit against the oracle where the warp's range
+search can go wrong: a single photon, ranges that hold more photons than the
+kernel keeps for its second pass, leaves counted as a whole, query counts beside
+a block's."""
+import numpy as np
+import pytest
+import torch
+
+from mnrt_b200 import _lib as L
+from mnrt_b200 import gen
+from mnrt_b200.photon_map import PhotonMap
+from tests.test_gpu_parity import format_errors, radiance_errors
+
+pytestmark = pytest.mark.gpu
+
+
+def to_dev(a, dev):
+    return torch.from_numpy(np.ascontiguousarray(a)).to(dev)
+
+
+@pytest.mark.parametrize("n,nq,k,r,iters,filt", [
+    (1, 40, 3, 0.2, 2, "box"),
+    (700, 1025, 128, 0.5, 0, "cone"),            # no refinement: ranges beyond the kept photons
+    (30000, 3001, 20, 0.3, 1, "epanechnikov"),   # node estimates; bins counted a leaf at a time
+    (30000, 999, 128, 0.1, 5, "cone"),
+])
+def test_compat_ranges(cuda, oracle_mod, n, nq, k, r, iters, filt):
+    ph = gen.photons(n, seed=n, caustic_frac=0.5)
+    q = gen.queries(nq, seed=nq, cluster_frac=0.5)
+    pm = PhotonMap(n, global_q_radius_max=r, knn_target_count=k)
+    pm.set_tuning(leaf_size=16)
+    pm.build(to_dev(ph.pos, cuda), to_dev(ph.pow, cuda))
+    qp, qn = to_dev(q.pos, cuda), to_dev(q.nrm, cuda)
+    out = pm.query(qp, qn, mode=L.PM_MODE_ZHOU_COMPAT, refine_iters=iters, filter=filt, min_found=8)
+    radii = pm.compute_query_radii(qp, refine_iters=iters)
+    torch.cuda.synchronize()
+    nodes, tpos, tpow = pm.export_tree()
+    o_radius, o_count, o_r2, o_rad = oracle_mod.compat(nodes, tpos, tpow, q.pos, q.nrm, k, r, iters, filt, 1.0, 8)
+    assert np.array_equal(radii.cpu().numpy(), o_radius)
+    assert np.array_equal(out["count"].cpu().numpy().view(np.uint32), o_count)
+    assert np.array_equal(out["r2"].cpu().numpy(), o_r2)
+    e = radiance_errors(out["rad"].cpu().numpy()[:, :3], o_rad)
+    assert e["max"] <= 1e-5, format_errors(e)
+    assert pm.info().device_errors == 0
