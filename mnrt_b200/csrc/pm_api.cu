@@ -46,7 +46,7 @@ struct pm_map {
     // photon-sized
     DevBuf pos, pow, inv, nodes, hdr;
     DevBuf keys0, keys1, vals0, vals1, scratch, kfirst, klast, ksplit, kkeep, krank, parent, arrive, nleaf, partials;
-    DevBuf wflag, wcnt, wfirst, wchild, wroot, wscan, rootmark;   // 32-wide tree
+    DevBuf wslot, wcnt, wfirst, wchild, wroot, wscan, rootmark;   // 32-wide tree
     // query-sized
     DevBuf qkeys0, qkeys1, qvals0, qvals1, qscratch, counter, fixq, qsorted;
     DevBuf stats;           // query counters (profiling level 2)
@@ -182,12 +182,12 @@ pm_status ensure_photon_capacity(pm_map* m, uint32_t n, cudaStream_t st) {
     ENSURE(arrive, (cap + 1) * sizeof(uint32_t));
     ENSURE(nleaf, (cap + 1) * sizeof(uint32_t));
     ENSURE(partials, (8 * 1184 + 16) * sizeof(uint32_t));
-    ENSURE(wflag, cap * sizeof(uint32_t));
+    ENSURE(wslot, (cap + 1) * 2 * sizeof(uint32_t));
     ENSURE(wcnt, cap * sizeof(uint32_t));
     ENSURE(wfirst, cap * sizeof(uint32_t));
     ENSURE(wchild, (cap + 1) * 2 * sizeof(ChildSlot));
     ENSURE(wroot, sizeof(ChildSlot));
-    ENSURE(wscan, wide_scan_words((uint32_t)cap) * sizeof(uint32_t));
+    ENSURE(wscan, 4 * sizeof(uint32_t));
     ENSURE(rootmark, (cap + 1) * sizeof(uint32_t));
 #undef ENSURE
     m->cap_photons = (uint32_t)cap;
@@ -250,7 +250,7 @@ MapView view_of(pm_map* m) {
 
 WideBuffers wide_of(pm_map* m) {
     WideBuffers w;
-    w.wflag = P<uint32_t>(m->wflag); w.wcnt = P<uint32_t>(m->wcnt);
+    w.wslot = P<uint32_t>(m->wslot); w.wcnt = P<uint32_t>(m->wcnt);
     w.wfirst = P<uint32_t>(m->wfirst); w.wchild = P<ChildSlot>(m->wchild); w.wroot = P<ChildSlot>(m->wroot);
     w.scratch = P<uint32_t>(m->wscan);
     return w;
@@ -329,7 +329,7 @@ pm_status pm_destroy(pm_map* m) {
     if (!m) return PM_ERR_INVALID;
     DevBuf* all[] = {&m->pos, &m->pow, &m->inv, &m->nodes, &m->hdr, &m->keys0, &m->keys1, &m->vals0, &m->vals1,
                      &m->scratch, &m->kfirst, &m->klast, &m->ksplit, &m->kkeep, &m->krank, &m->parent,
-                     &m->arrive, &m->nleaf, &m->partials, &m->wflag, &m->wcnt, &m->wfirst,
+                     &m->arrive, &m->nleaf, &m->partials, &m->wslot, &m->wcnt, &m->wfirst,
                      &m->wchild, &m->wroot, &m->wscan, &m->rootmark, &m->qkeys0, &m->qkeys1, &m->qvals0, &m->qvals1,
                      &m->qscratch, &m->counter, &m->fixq, &m->qsorted, &m->stats, &m->bvals, &m->bvals1, &m->bkeys0, &m->bkeys1, &m->blong,
                      &m->bscratch, &m->qrec, &m->seg_start, &m->seg_end, &m->acc, &m->rnbr,
@@ -1337,10 +1337,12 @@ pm_status batch_build_device(pm_batch* b, const float* d_pos4, const float* d_po
     uint64_t* keys[2] = {bb.keys[0], bb.keys[1]};
     uint32_t* vals[2] = {bb.vals[0], bb.vals[1]};
     const SortGather g{pos, pw, format, P<float4>(m->pos), P<float4>(m->pow), P<uint32_t>(m->inv)};
-    const int cur = n > 1 ? radix_sort_pairs(keys, vals, n, kMortonBits + map_id_bits(maps), bb.scratch, st, &nl, &g) : 0;
+    const bool fuse = n > 1 && n <= kGatherInSortMax;
+    const int cur = n > 1 ? radix_sort_pairs(keys, vals, n, kMortonBits + map_id_bits(maps), bb.scratch, st, &nl,
+                                             fuse ? &g : nullptr) : 0;
     nl += build_from_sorted(pos, pw, n, format, m->leaf_size, keys[cur], vals[cur], P<float4>(m->pos),
                             P<float4>(m->pow), P<uint32_t>(m->inv), P<Node>(m->nodes), P<MapHeader>(m->hdr), bb, st,
-                            n > 1);
+                            fuse);
     nl += batch_roots(P<uint32_t>(b->ph_off), maps, n, m->leaf_size, P<float4>(m->pos), P<Node>(m->nodes), bb,
                       P<BatchGeom>(b->geom), st);
     nl += batch_wide(n, maps, P<Node>(m->nodes), P<uint32_t>(m->parent), P<MapHeader>(m->hdr), P<uint32_t>(m->rootmark),

@@ -159,8 +159,8 @@ __device__ __forceinline__ void slot_box(const float4* __restrict__ pos, uint32_
 __global__ void k_batch_roots(const uint32_t* __restrict__ off, uint32_t m, uint32_t n, uint32_t leaf_size,
                               const float4* __restrict__ pos, const Node* __restrict__ nodes,
                               const uint32_t* __restrict__ kfirst, const uint32_t* __restrict__ klast,
-                              const uint32_t* __restrict__ krank, const uint32_t* __restrict__ parent,
-                              BatchGeom* __restrict__ geom) {
+                              const uint32_t* __restrict__ kkeep, const uint32_t* __restrict__ krank,
+                              const uint32_t* __restrict__ parent, BatchGeom* __restrict__ geom) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
     const uint32_t s = off[i], e = off[i + 1];
@@ -171,8 +171,8 @@ __global__ void k_batch_roots(const uint32_t* __restrict__ off, uint32_t m, uint
         slot.cnt = e - s;
     } else if (e > s) {
         uint32_t r = kInvalid;
-        if (s < n - 1 && kfirst[s] == s && klast[s] == e - 1) r = s;
-        else if (e - 1 < n - 1 && kfirst[e - 1] == s && klast[e - 1] == e - 1) r = e - 1;
+        if (s < n - 1 && kkeep[s] && kfirst[s] == s && klast[s] == e - 1) r = s;
+        else if (e - 1 < n - 1 && kkeep[e - 1] && kfirst[e - 1] == s && klast[e - 1] == e - 1) r = e - 1;
         if (r != kInvalid) {
             const uint32_t id = 1 + krank[r];
             if (id == 1) {
@@ -249,8 +249,8 @@ int batch_query_keys(const float4* qpos, const uint32_t* q_off, uint32_t m, uint
 
 int batch_roots(const uint32_t* ph_off, uint32_t m, uint32_t n, uint32_t leaf_size, const float4* pos,
                 const Node* nodes, const BuildBuffers& bb, BatchGeom* geom, cudaStream_t st) {
-    k_batch_roots<<<(m + 127) / 128, 128, 0, st>>>(ph_off, m, n, leaf_size, pos, nodes, bb.kfirst, bb.klast, bb.krank,
-                                                    bb.parent, geom);
+    k_batch_roots<<<(m + 127) / 128, 128, 0, st>>>(ph_off, m, n, leaf_size, pos, nodes, bb.kfirst, bb.klast, bb.kkeep,
+                                                    bb.krank, bb.parent, geom);
     return 1;
 }
 

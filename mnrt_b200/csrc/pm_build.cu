@@ -26,17 +26,17 @@
 //                     internal node, leaf boxes computed from their photons
 //   8. k_refit        bottom-up child boxes (atomic arrival counters; boxes
 //                     are min/max so the result is order independent)
+#include <algorithm>
+
 #include "pm_internal.h"
+#include "pm_sort_small.cuh"
 
 namespace pm {
 
 constexpr int kBoundsThreads = 256;
 constexpr int kBoundsBlocksMax = 1184;   // 8 per SM on 148 SMs
 constexpr int kLeafBoxBlocks = 1184;     // 8 blocks of 8 warps per SM, grid-stride over the nodes
-
-// The wide tree's child-count scan in WideBuffers::scratch: ticket, total,
-// one uint64 look-back word per tile of 256 nodes.
-size_t wide_scan_words(uint32_t n) { return 2 + 2 * (size_t)((n + 255) / 256); }
+constexpr uint32_t kWideEmitBlocks = 592;   // 4 blocks per SM, grid-stride over the child slots
 
 __device__ __forceinline__ float warp_min(float v) {
 #pragma unroll
@@ -165,21 +165,33 @@ __device__ __forceinline__ int delta(const uint64_t* __restrict__ keys, int64_t 
     return 64 + __clz((uint32_t)i ^ (uint32_t)j);
 }
 
-// Thread per radix-tree node i (Karras 2012): direction, range [first, last],
-// split, and the keep flag (more than leaf_size photons).
-__global__ void k_radix_tree(const uint64_t* __restrict__ keys, uint32_t n, uint32_t leaf_size,
-                             uint32_t* __restrict__ kfirst, uint32_t* __restrict__ klast,
-                             uint32_t* __restrict__ ksplit, uint32_t* __restrict__ kkeep) {
+constexpr int kTreeThreads = 256;
+constexpr uint32_t kTreeScanBlocks = 1024;   // block counts k_emit scans itself (4 per thread)
+
+__device__ __forceinline__ bool radix_tree_node(const uint64_t* __restrict__ keys, uint32_t n, uint32_t leaf_size,
+                                                uint32_t* __restrict__ kfirst, uint32_t* __restrict__ klast,
+                                                uint32_t* __restrict__ ksplit, uint32_t* __restrict__ kkeep) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t nn = n;
-    if (i >= nn - 1) return;
+    if (i >= nn - 1) return false;
     const int d = (delta(keys, nn, i, i + 1) > delta(keys, nn, i, i - 1)) ? 1 : -1;
     const int dmin = delta(keys, nn, i, i - d);
-    int64_t lmax = 2;
-    while (delta(keys, nn, i, i + lmax * d) > dmin) lmax <<= 1;
-    int64_t l = 0;
-    for (int64_t t = lmax >> 1; t >= 1; t >>= 1)
-        if (delta(keys, nn, i, i + (l + t) * d) > dmin) l += t;
+    // A node of at most leaf_size photons is dropped: one look at the key
+    // leaf_size further on tells, and all but about 2 / leaf_size of the nodes
+    // end here without their searches (20.5M photons: 698 -> 380 us; 1M: 47 -> 38).
+    // What is left is the latency of the kept nodes' searches, a lane or two a warp.
+    int64_t l = (int64_t)leaf_size;
+    if (!(delta(keys, nn, i, i + l * d) > dmin)) {
+        kkeep[i] = 0u;
+        return false;
+    }
+    int64_t over = 2 * l;   // l is within the range, over past its end
+    while (delta(keys, nn, i, i + over * d) > dmin) { l = over; over <<= 1; }
+    while (over - l > 1) {
+        const int64_t mid = (l + over) >> 1;
+        if (delta(keys, nn, i, i + mid * d) > dmin) l = mid;
+        else over = mid;
+    }
     const int64_t j = i + l * d;
     const int dnode = delta(keys, nn, i, j);
     int64_t s = 0, t = l;
@@ -192,7 +204,34 @@ __global__ void k_radix_tree(const uint64_t* __restrict__ keys, uint32_t n, uint
     kfirst[i] = (uint32_t)first;
     klast[i] = (uint32_t)last;
     ksplit[i] = (uint32_t)gamma;
-    kkeep[i] = (last - first + 1 > (int64_t)leaf_size) ? 1u : 0u;
+    kkeep[i] = 1u;
+    return true;
+}
+
+// Thread per radix-tree node i (Karras 2012): the keep flag (more than
+// leaf_size photons) and a kept node's range [first, last] and split.  kScan (small maps):
+// also the keep flags' exclusive scan within the block and the block's count,
+// which k_emit turns into ranks, so no scan is launched.  clear: words to zero
+// for a later launch (fewer than there are threads), or nullptr.
+template <bool kScan>
+__global__ void __launch_bounds__(kTreeThreads) k_radix_tree(const uint64_t* __restrict__ keys, uint32_t n, uint32_t leaf_size,
+                             uint32_t* __restrict__ kfirst, uint32_t* __restrict__ klast,
+                             uint32_t* __restrict__ ksplit, uint32_t* __restrict__ kkeep,
+                             uint32_t* __restrict__ krank, uint32_t* __restrict__ counts,
+                             uint32_t* __restrict__ clear, uint32_t clear_words) {
+    {
+        const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+        if (t < clear_words) clear[t] = 0u;
+    }
+    const bool keep = radix_tree_node(keys, n, leaf_size, kfirst, klast, ksplit, kkeep);
+    if constexpr (kScan) {
+        __shared__ uint32_t s_warp[32];
+        const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+        uint32_t total;
+        const uint32_t ex = block_exclusive_scan(keep ? 1u : 0u, s_warp, total);
+        if (i + 1 < n) krank[i] = ex;
+        if (threadIdx.x == 0) counts[blockIdx.x] = total;
+    }
 }
 
 __device__ __forceinline__ void leaf_box(const float4* __restrict__ pos, uint32_t first, uint32_t cnt, ChildSlot& s) {
@@ -215,16 +254,38 @@ __device__ __forceinline__ ChildSlot empty_slot() {
     return s;
 }
 
-// Thread per radix-tree node; kept nodes write their compacted node.
-__global__ void k_emit(const float4* __restrict__ pos, uint32_t n, uint32_t leaf_size,
+// Thread per radix-tree node; kept nodes write their compacted node.  A node's
+// rank among the kept ones is krank (total: their count), or with counts
+// (k_radix_tree<true>) krank plus the counts of the blocks before its own.
+__global__ void __launch_bounds__(kTreeThreads) k_emit(const float4* __restrict__ pos, uint32_t n, uint32_t leaf_size,
                        const uint32_t* __restrict__ kfirst, const uint32_t* __restrict__ klast,
                        const uint32_t* __restrict__ ksplit, const uint32_t* __restrict__ kkeep,
-                       const uint32_t* __restrict__ krank, const uint32_t* __restrict__ total, Node* __restrict__ nodes,
+                       const uint32_t* __restrict__ krank, const uint32_t* __restrict__ total_in,
+                       const uint32_t* __restrict__ counts, uint32_t nblocks, Node* __restrict__ nodes,
                        uint32_t* __restrict__ parent, uint32_t* __restrict__ arrive, uint32_t* __restrict__ nleaf,
                        MapHeader* hdr) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ uint32_t s_before[kTreeScanBlocks], s_warp[32];
+    uint32_t kept = 0;
+    if (counts) {
+        uint32_t c[4], sum = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t b = threadIdx.x * 4u + k;
+            c[k] = b < nblocks ? counts[b] : 0u;
+            sum += c[k];
+        }
+        uint32_t run = block_exclusive_scan(sum, s_warp, kept);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            s_before[threadIdx.x * 4u + k] = run;
+            run += c[k];
+        }
+        __syncthreads();
+    }
+    auto rank_of = [&](uint32_t c) { return krank[c] + (counts ? s_before[c / kTreeThreads] : 0u); };
     if (i == 0) {
-        const uint32_t m = (n > 1) ? *total : 0u;
+        const uint32_t m = counts ? kept : ((n > 1) ? *total_in : 0u);
         hdr->num_nodes = m;
         Node sr;
         sr.c[1] = empty_slot();
@@ -244,7 +305,7 @@ __global__ void k_emit(const float4* __restrict__ pos, uint32_t n, uint32_t leaf
         nodes[0] = sr;
     }
     if (n < 2 || i >= (uint64_t)n - 1 || !kkeep[i]) return;
-    const uint32_t id = 1 + krank[i];
+    const uint32_t id = 1 + rank_of((uint32_t)i);
     const uint32_t first = kfirst[i], last = klast[i], gamma = ksplit[i];
     Node nd;
     uint32_t leaves = 0;
@@ -261,7 +322,7 @@ __global__ void k_emit(const float4* __restrict__ pos, uint32_t n, uint32_t leaf
             ++leaves;
         } else {
             const uint32_t c = side ? gamma + 1 : gamma;   // radix-tree index of the internal child
-            const uint32_t cid = 1 + krank[c];
+            const uint32_t cid = 1 + rank_of(c);
             s = empty_slot();
             s.ref = cid;
             s.cnt = 0;
@@ -381,44 +442,56 @@ void scale_flux(float4* pw, uint32_t n, float scale, MapHeader* hdr, cudaStream_
 // nodes, refit.  keys/vals are the sorted (code, caller index) pairs; any
 // code whose prefix separates groups (e.g. a map id in the top bits) yields
 // one subtree per group.
-// k_refit_wide_count is defined with the wide tree below.
+// k_refit_wide_count and k_wide_emit are defined with the wide tree below.
 __global__ void k_refit_wide_count(Node* nodes, const uint32_t* __restrict__ parent, uint32_t* arrive,
                                    const uint32_t* __restrict__ nleaf, const MapHeader* __restrict__ hdr,
                                    uint32_t max_nodes, uint32_t refit_blocks, uint32_t bound,
-                                   uint32_t* __restrict__ wflag, uint32_t* __restrict__ wcnt,
-                                   uint32_t* __restrict__ wfirst, uint32_t* scan, uint32_t* err);
-__global__ void k_wide_emit(const Node* __restrict__ nodes, const uint32_t* __restrict__ rootmark,
-                            const uint32_t* __restrict__ wflag, const uint32_t* __restrict__ wcnt,
-                            const uint32_t* __restrict__ wfirst, const MapHeader* __restrict__ hdr, uint32_t bound,
-                            ChildSlot* __restrict__ wchild, ChildSlot* __restrict__ wroot);
+                                   uint32_t* __restrict__ wcnt, uint32_t* __restrict__ wfirst,
+                                   uint32_t* __restrict__ wslot, uint32_t* __restrict__ total);
+__global__ void k_wide_emit(const Node* __restrict__ nodes, const uint32_t* __restrict__ wslot,
+                            const uint32_t* __restrict__ wcnt, const uint32_t* __restrict__ wfirst,
+                            const uint32_t* __restrict__ total, ChildSlot* __restrict__ wchild,
+                            ChildSlot* __restrict__ wroot);
 
 int build_from_sorted(const float4* in_pos, const float4* in_pow, uint32_t n, int format, uint32_t leaf_size,
                       const uint64_t* keys, const uint32_t* vals, float4* out_pos, float4* out_pow, uint32_t* inv,
                       Node* nodes, MapHeader* hdr, const BuildBuffers& bb, cudaStream_t st, bool gathered,
                       const WideBuffers* wide) {
-    const uint32_t tb = 256;
+    const uint32_t tb = kTreeThreads;
     if (n > 0) {
         if (!gathered) k_gather<<<(n + tb - 1) / tb, tb, 0, st>>>(in_pos, in_pow, vals, n, format, out_pos, out_pow, inv);
         const int ng = gathered ? 0 : 1;
         if (n > 1) {
             const uint32_t ni = n - 1, gi = (ni + tb - 1) / tb;
-            // the keep flags' exclusive scan (a single-pass scan with look-back inside
-            // k_radix_tree measured 87 us against 46 + 13 us: one slow tile holds up
-            // every later one, where separate kernels let blocks finish independently)
-            k_radix_tree<<<gi, tb, 0, st>>>(keys, n, leaf_size, bb.kfirst, bb.klast, bb.ksplit, bb.kkeep);
             uint32_t* total = bb.scratch + sort_scratch_words(n);
-            const int ns = exclusive_scan(bb.kkeep, bb.krank, ni, total + 1, total, st);
+            uint32_t* clear = wide ? wide->scratch : nullptr;
+            const uint32_t clear_words = wide ? 1u : 0u;
+            int ns = 0;
+            // The keep flags' ranks.  Up to 262,144 photons k_emit sums the block
+            // counts itself; above, three scan launches (a single-pass scan with
+            // look-back inside k_radix_tree measured 87 us against 46 + 13 us: one
+            // slow tile holds up every later one, where separate kernels let blocks
+            // finish independently).  The batch's roots read whole ranks, so they
+            // take the scan.
+            const bool own = wide && gi <= kTreeScanBlocks;
+            uint32_t* counts = bb.scratch;   // the sort's scratch is free, and holds n / 8 words at least
+            if (own) {
+                k_radix_tree<true><<<gi, tb, 0, st>>>(keys, n, leaf_size, bb.kfirst, bb.klast, bb.ksplit, bb.kkeep, bb.krank,
+                                                      counts, clear, clear_words);
+            } else {
+                k_radix_tree<false><<<gi, tb, 0, st>>>(keys, n, leaf_size, bb.kfirst, bb.klast, bb.ksplit, bb.kkeep, bb.krank,
+                                                       nullptr, clear, clear_words);
+                ns = exclusive_scan(bb.kkeep, bb.krank, ni, total + 1, total, st);
+            }
             k_emit<<<gi, tb, 0, st>>>(out_pos, n, leaf_size, bb.kfirst, bb.klast, bb.ksplit, bb.kkeep, bb.krank,
-                                      total, nodes, bb.parent, bb.arrive, bb.nleaf, hdr);
+                                      total, own ? counts : nullptr, gi, nodes, bb.parent, bb.arrive, bb.nleaf, hdr);
             k_leaf_boxes<<<kLeafBoxBlocks, 256, 0, st>>>(out_pos, nodes, hdr);
             if (wide) {   // the single-map build: refit and the wide tree's counts in one launch
                 const uint32_t wgrid = (ni + 255u) / 256u;
-                cudaMemsetAsync(wide->scratch, 0, wide_scan_words(n) * sizeof(uint32_t), st);
                 k_refit_wide_count<<<gi + wgrid, tb, 0, st>>>(nodes, bb.parent, bb.arrive, bb.nleaf, hdr, n, gi, ni,
-                                                             wide->wflag, wide->wcnt, wide->wfirst, wide->scratch,
-                                                             &hdr->errors);
-                k_wide_emit<<<wgrid, 256, 0, st>>>(nodes, nullptr, wide->wflag, wide->wcnt, wide->wfirst, hdr, ni,
-                                                   wide->wchild, wide->wroot);
+                                                              wide->wcnt, wide->wfirst, wide->wslot, wide->scratch);
+                k_wide_emit<<<std::min(wgrid, kWideEmitBlocks), 256, 0, st>>>(nodes, wide->wslot, wide->wcnt, wide->wfirst,
+                                                                              wide->scratch, wide->wchild, wide->wroot);
                 return ng + 6 + ns;
             }
             k_refit<<<gi, tb, 0, st>>>(nodes, bb.parent, bb.arrive, bb.nleaf, hdr, n);
@@ -426,34 +499,132 @@ int build_from_sorted(const float4* in_pos, const float4* in_pow, uint32_t n, in
         }
     }
     k_emit<<<1, 32, 0, st>>>(out_pos, n, leaf_size, bb.kfirst, bb.klast, bb.ksplit, bb.kkeep, bb.krank, nullptr,
-                             nodes, bb.parent, bb.arrive, bb.nleaf, hdr);
+                             nullptr, 0u, nodes, bb.parent, bb.arrive, bb.nleaf, hdr);
     return n > 0 ? 2 : 1;
+}
+
+// Small maps (up to kSmallSortMax photons): bounds, Morton codes, sort and the
+// move into tree order in one launch of one cluster, in place of two kernels,
+// 15 sort launches and two clears.  The same values and the same order as
+// k_bounds, k_morton and the radix sort give.
+template <int R>
+__global__ void __launch_bounds__(kSmallSortThreads, 1) k_small_build(const float4* __restrict__ pos,
+                                                                      const float4* __restrict__ pw, uint32_t n,
+                                                                      SortGather g, uint64_t* __restrict__ keys_out,
+                                                                      MapHeader* hdr) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ float s_v[kSmallSortWarps][8];
+    __shared__ float s_part[8];   // this block's bounds, read by the cluster
+    __shared__ float s_all[8];
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t first = cluster.block_rank() * (uint32_t)(kSmallSortThreads * R) + warp * 32u * R + lane;
+    float v[7] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY, 0.0f};
+    uint32_t bad = 0;
+    float4 p[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t i = first + 32u * r;
+        p[r] = i < n ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i >= n) continue;
+        const float4 w = pw[i];
+        if (!(isfinite(p[r].x) && isfinite(p[r].y) && isfinite(p[r].z))) { bad = 1; continue; }
+        v[0] = fminf(v[0], p[r].x); v[1] = fminf(v[1], p[r].y); v[2] = fminf(v[2], p[r].z);
+        v[3] = fmaxf(v[3], p[r].x); v[4] = fmaxf(v[4], p[r].y); v[5] = fmaxf(v[5], p[r].z);
+        v[6] = fmaxf(v[6], fmaxf(fmaxf(fabsf(w.x), fabsf(w.y)), fabsf(w.z)));
+    }
+    // warp, block, cluster: one row of eight values per reduced unit
+    auto reduce_row = [&](float* out) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) { v[a] = warp_min(v[a]); v[a + 3] = warp_max(v[a + 3]); }
+        v[6] = warp_max(v[6]);
+        bad = __any_sync(0xffffffffu, bad != 0) ? 1u : 0u;
+        if (lane == 0) {
+#pragma unroll
+            for (int a = 0; a < 7; ++a) out[a] = v[a];
+            out[7] = __uint_as_float(bad);
+        }
+    };
+    auto take_row = [&](const float* in, bool have) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) { v[a] = have ? in[a] : INFINITY; v[a + 3] = have ? in[a + 3] : -INFINITY; }
+        v[6] = have ? in[6] : 0.0f;
+        bad = have ? __float_as_uint(in[7]) : 0u;
+    };
+    reduce_row(s_v[warp]);
+    __syncthreads();
+    if (warp == 0) {
+        take_row(s_v[lane], true);
+        reduce_row(s_part);
+    }
+    cluster.sync();
+    if (warp == 0) {
+        const bool have = lane < cluster.num_blocks();
+        take_row(cluster.map_shared_rank(&s_part[0], have ? lane : 0u), have);
+        reduce_row(s_all);
+    }
+    __syncthreads();
+    if (cluster.block_rank() == 0 && threadIdx.x == 0) {
+        for (int a = 0; a < 3; ++a) { hdr->lo[a] = s_all[a]; hdr->hi[a] = s_all[a + 3]; }
+        hdr->max_power = s_all[6];
+        hdr->fix_scale = fix_scale_of(s_all[6]);
+        hdr->n = n;
+        hdr->errors = __float_as_uint(s_all[7]) ? kErrNonFinite : 0u;
+    }
+    const float ext = fmaxf(fmaxf(__fsub_rn(s_all[3], s_all[0]), __fsub_rn(s_all[4], s_all[1])),
+                            __fsub_rn(s_all[5], s_all[2]));
+    const float scale = (ext > 0.0f && isfinite(ext)) ? __fdiv_rn(65536.0f, ext) : 0.0f;
+    uint64_t key[R];
+    uint32_t val[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        key[r] = morton39(p[r].x, p[r].y, p[r].z, s_all, scale);
+        val[r] = first + 32u * r;
+    }
+    small_sort<uint64_t, R>(key, val, n, kMortonBits, smem, [&](uint32_t dst, uint64_t k, uint32_t src) {
+        keys_out[dst] = k;
+        const float4 q = g.in_pos[src];
+        const float4 w = g.in_pow[src];
+        const uint32_t dir = (g.format == 0) ? spherical_to_oct(q.w, w.w) : __float_as_uint(w.w);
+        g.out_pos[dst] = make_float4(q.x, q.y, q.z, __uint_as_float(src));
+        g.out_pow[dst] = make_float4(w.x, w.y, w.z, __uint_as_float(dir));
+        g.inv[src] = dst;
+    });
 }
 
 int build_map(const float4* in_pos, const float4* in_pow, uint32_t n, int format, uint32_t leaf_size,
               float4* out_pos, float4* out_pow, uint32_t* inv, Node* nodes, MapHeader* hdr, const BuildBuffers& bb,
               const WideBuffers& wide, cudaStream_t st, cudaEvent_t sort_done) {
     int nl = 0;
-    const uint32_t nb = (uint32_t)((n + kBoundsThreads - 1) / kBoundsThreads);
-    const uint32_t bblocks = nb < 1 ? 1 : (nb > (uint32_t)kBoundsBlocksMax ? (uint32_t)kBoundsBlocksMax : nb);
-    cudaMemsetAsync(&hdr->errors, 0, sizeof(uint32_t), st);
-    cudaMemsetAsync(bb.partials + 8 * bblocks, 0, sizeof(uint32_t), st);
-    k_bounds<<<bblocks, kBoundsThreads, 0, st>>>(in_pos, in_pow, n, reinterpret_cast<float*>(bb.partials), hdr);
-    ++nl;
     uint64_t* keys[2] = {bb.keys[0], bb.keys[1]};
     uint32_t* vals[2] = {bb.vals[0], bb.vals[1]};
     int cur = 0;
-    if (n > 0) {
-        const uint32_t tb = 256;
-        k_morton<<<(n + tb - 1) / tb, tb, 0, st>>>(in_pos, n, hdr, bb.keys[0], bb.vals[0]);
+    // the last sort pass moves the photons into tree order (n >= 2; one photon is not sorted)
+    const SortGather g{in_pos, in_pow, format, out_pos, out_pow, inv};
+    const bool fuse = n > 1 && n <= kGatherInSortMax;
+    if (n > 1 && n <= kSmallSortMax) {
+        if (n <= kSmallSortMax / 4) launch_small_sort<uint64_t, 1>(k_small_build<1>, n, st, in_pos, in_pow, n, g, keys[0], hdr);
+        else if (n <= kSmallSortMax / 2) launch_small_sort<uint64_t, 2>(k_small_build<2>, n, st, in_pos, in_pow, n, g, keys[0], hdr);
+        else launch_small_sort<uint64_t, 4>(k_small_build<4>, n, st, in_pos, in_pow, n, g, keys[0], hdr);
         ++nl;
-        // the last pass moves the photons into tree order (n >= 2; one photon is not sorted)
-        const SortGather g{in_pos, in_pow, format, out_pos, out_pow, inv};
-        cur = radix_sort_pairs(keys, vals, n, kMortonBits, bb.scratch, st, &nl, n > 1 ? &g : nullptr);
+    } else {
+        const uint32_t nb = (uint32_t)((n + kBoundsThreads - 1) / kBoundsThreads);
+        const uint32_t bblocks = nb < 1 ? 1 : (nb > (uint32_t)kBoundsBlocksMax ? (uint32_t)kBoundsBlocksMax : nb);
+        cudaMemsetAsync(&hdr->errors, 0, sizeof(uint32_t), st);
+        cudaMemsetAsync(bb.partials + 8 * bblocks, 0, sizeof(uint32_t), st);
+        k_bounds<<<bblocks, kBoundsThreads, 0, st>>>(in_pos, in_pow, n, reinterpret_cast<float*>(bb.partials), hdr);
+        ++nl;
+        if (n > 0) {
+            const uint32_t tb = 256;
+            k_morton<<<(n + tb - 1) / tb, tb, 0, st>>>(in_pos, n, hdr, bb.keys[0], bb.vals[0]);
+            ++nl;
+            cur = radix_sort_pairs(keys, vals, n, kMortonBits, bb.scratch, st, &nl, fuse ? &g : nullptr);
+        }
     }
     if (sort_done) cudaEventRecord(sort_done, st);
     nl += build_from_sorted(in_pos, in_pow, n, format, leaf_size, keys[cur], vals[cur], out_pos, out_pow, inv, nodes,
-                            hdr, bb, st, n > 1, &wide);
+                            hdr, bb, st, fuse, &wide);
     if (n <= 1) nl += build_wide(n, nodes, bb.parent, nullptr, hdr, wide, st);   // the start slot only
     return nl;
 }
@@ -515,94 +686,77 @@ __device__ uint32_t wide_expand_warp(const Node* __restrict__ nodes, const uint3
     return count;
 }
 
-// Block of 8 warps per 256 consecutive compacted nodes, taken by ticket: each
-// lane marks its node as wide when the node lies a multiple of kWideLevels
-// below its root (node 1, or a node marked in rootmark), the warps expand
-// their wide nodes to count the children, and the block's exclusive scan of
-// the counts plus a decoupled look-back gives every wide node its first
-// child slot (one launch for flags, counts and scan).  scan: [0] ticket, [1]
-// total child slots (last tile), look-back words from word 2; cleared before.
+// Block of 8 warps per 256 consecutive compacted nodes: each lane marks its
+// node as wide when the node lies a multiple of kWideLevels below its root
+// (node 1, or a node marked in rootmark); the block's wide nodes are then
+// expanded by its warps in turn, and each takes its child slots' places from
+// one counter (where they lie does not matter to the traversal, which only
+// follows first indices) and lists them there: slot << 1 | wide.
 __device__ __forceinline__ void wide_count_block(const Node* __restrict__ nodes, const uint32_t* __restrict__ parent,
                                                  const uint32_t* __restrict__ rootmark,
-                                                 const MapHeader* __restrict__ hdr, uint32_t bound,
-                                                 uint32_t* __restrict__ wflag, uint32_t* __restrict__ wcnt,
-                                                 uint32_t* __restrict__ wfirst, uint32_t* scan, uint32_t* err) {
+                                                 const MapHeader* __restrict__ hdr, uint32_t bound, uint32_t block,
+                                                 uint32_t* __restrict__ wcnt, uint32_t* __restrict__ wfirst,
+                                                 uint32_t* __restrict__ wslot, uint32_t* __restrict__ total) {
     __shared__ uint32_t s_buf[8][64];
-    __shared__ uint32_t s_tile, s_warp[32];
-    __shared__ uint64_t s_before;
-    if (threadIdx.x == 0) s_tile = atomicAdd(&scan[0], 1u);
-    __syncthreads();
+    __shared__ uint32_t s_node[256], s_wide;
     const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-    const uint32_t t0 = s_tile * 256u + wib * 32u;
     const uint32_t m = hdr->num_nodes;
-    const uint32_t t = t0 + lane;
-    bool wide = false;
+    const uint32_t t = block * 256u + threadIdx.x;
+    if (block * 256u >= m) return;   // the whole block
+    if (threadIdx.x == 0) s_wide = 0;
+    __syncthreads();
     if (t < m && t < bound) {
         uint32_t c = t + 1, d = 0;
         while (!is_marked_root(rootmark, c) && d < 4096) { c = parent[c] >> 1; ++d; }
-        wide = d % kWideLevels == 0;
-    }
-    uint32_t mine = 0;
-    uint32_t todo = __ballot_sync(0xffffffffu, wide);
-    while (todo) {
-        const uint32_t b = __ffs(todo) - 1;
-        todo &= todo - 1;
-        uint32_t slot, state;
-        const uint32_t c = wide_expand_warp(nodes, rootmark, t0 + b + 1u, lane, s_buf[wib], slot, state);
-        if (lane == b) mine = c;
-    }
-    uint32_t total;
-    const uint32_t ex = block_exclusive_scan(mine, s_warp, total);
-    if (threadIdx.x < 32) {
-        const uint64_t b = warp_lookback_exclusive(reinterpret_cast<uint64_t*>(scan + 2), s_tile, total, err);
-        if (threadIdx.x == 0) s_before = b;
+        if (d % kWideLevels == 0) s_node[atomicAdd(&s_wide, 1u)] = t;
     }
     __syncthreads();
-    if (t < bound) {
-        wflag[t] = wide ? 1u : 0u;
-        wcnt[t] = mine;
-        wfirst[t] = (uint32_t)s_before + ex;
+    for (uint32_t w = wib; w < s_wide; w += 8) {
+        uint32_t slot, state, first = 0;
+        const uint32_t j = s_node[w];
+        const uint32_t c = wide_expand_warp(nodes, rootmark, j + 1u, lane, s_buf[wib], slot, state);
+        if (lane == 0) first = atomicAdd(total, c);
+        first = __shfl_sync(0xffffffffu, first, 0);
+        if (lane == 0) { wcnt[j] = c; wfirst[j] = first; }
+        if (lane < c) wslot[first + lane] = (slot << 1) | (state == kItemWide ? 1u : 0u);
     }
-    if (threadIdx.x == 0 && s_tile + 1 == (bound + 255u) / 256u) scan[1] = (uint32_t)s_before + total;
 }
 
 __global__ void __launch_bounds__(256) k_wide_count(const Node* __restrict__ nodes, const uint32_t* __restrict__ parent,
                                                      const uint32_t* __restrict__ rootmark,
                                                      const MapHeader* __restrict__ hdr, uint32_t bound,
-                                                     uint32_t* __restrict__ wflag, uint32_t* __restrict__ wcnt,
-                                                     uint32_t* __restrict__ wfirst, uint32_t* scan, uint32_t* err) {
-    wide_count_block(nodes, parent, rootmark, hdr, bound, wflag, wcnt, wfirst, scan, err);
+                                                     uint32_t* __restrict__ wcnt, uint32_t* __restrict__ wfirst,
+                                                     uint32_t* __restrict__ wslot, uint32_t* __restrict__ total) {
+    wide_count_block(nodes, parent, rootmark, hdr, bound, blockIdx.x, wcnt, wfirst, wslot, total);
 }
 
-// The refit and the wide tree's counts in one launch: they are independent
-// (the counts read only the tree's structure, which k_emit wrote; the refit
-// writes only boxes), and both are latency-bound walks along root-to-leaf
-// paths, so blocks [0, refit_blocks) climb while the others count.  The
-// counting blocks take their tiles by ticket and wait only on each other.
+// The refit and the wide tree's shape in one launch: they are independent (the
+// counts read only the tree's structure, which k_emit wrote; the refit writes
+// only boxes), and both are latency-bound walks along root-to-leaf paths, so
+// blocks [0, refit_blocks) climb while the others count.
 __global__ void __launch_bounds__(256) k_refit_wide_count(Node* nodes, const uint32_t* __restrict__ parent,
                                                            uint32_t* arrive, const uint32_t* __restrict__ nleaf,
                                                            const MapHeader* __restrict__ hdr, uint32_t max_nodes,
                                                            uint32_t refit_blocks, uint32_t bound,
-                                                           uint32_t* __restrict__ wflag, uint32_t* __restrict__ wcnt,
-                                                           uint32_t* __restrict__ wfirst, uint32_t* scan,
-                                                           uint32_t* err) {
+                                                           uint32_t* __restrict__ wcnt, uint32_t* __restrict__ wfirst,
+                                                           uint32_t* __restrict__ wslot, uint32_t* __restrict__ total) {
     if (blockIdx.x < refit_blocks) {
         refit_thread(nodes, parent, arrive, nleaf, hdr, max_nodes, blockIdx.x * blockDim.x + threadIdx.x);
         return;
     }
-    wide_count_block(nodes, parent, nullptr, hdr, bound, wflag, wcnt, wfirst, scan, err);
+    wide_count_block(nodes, parent, nullptr, hdr, bound, blockIdx.x - refit_blocks, wcnt, wfirst, wslot, total);
 }
 
-// Warp per 32 consecutive compacted nodes: every wide node's child slots;
-// thread 0 of block 0 also writes the traversal's start slot (the
-// super-root's slot, pointing at the root wide node).
-__global__ void k_wide_emit(const Node* __restrict__ nodes, const uint32_t* __restrict__ rootmark,
-                            const uint32_t* __restrict__ wflag, const uint32_t* __restrict__ wcnt,
-                            const uint32_t* __restrict__ wfirst, const MapHeader* __restrict__ hdr, uint32_t bound,
-                            ChildSlot* __restrict__ wchild, ChildSlot* __restrict__ wroot) {
-    __shared__ uint32_t s_buf[8][64];
-    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+// Thread per listed child slot: the slot with its refitted box, a wide child
+// pointing at its own children.  (A warp per 32 nodes that expanded them again
+// took 31 us on 65,536 photons and 32 on 1M; this 5.)  Thread 0 also writes the
+// traversal's start slot (the super-root's, pointing at the root wide node).
+__global__ void __launch_bounds__(256) k_wide_emit(const Node* __restrict__ nodes, const uint32_t* __restrict__ wslot,
+                            const uint32_t* __restrict__ wcnt, const uint32_t* __restrict__ wfirst,
+                            const uint32_t* __restrict__ total, ChildSlot* __restrict__ wchild,
+                            ChildSlot* __restrict__ wroot) {
+    const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i0 == 0) {
         ChildSlot s = nodes[0].c[0];
         if (s.ref != kInvalid && s.cnt == 0) {
             s.ref = wfirst[0];
@@ -610,40 +764,29 @@ __global__ void k_wide_emit(const Node* __restrict__ nodes, const uint32_t* __re
         }
         *wroot = s;
     }
-    const uint32_t t0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32u;
-    if (t0 >= bound) return;
-    const uint32_t m = hdr->num_nodes;
-    const uint32_t t = t0 + lane;
-    uint32_t todo = __ballot_sync(0xffffffffu, t < m && t < bound && wflag[t]);
-    while (todo) {
-        const uint32_t b = __ffs(todo) - 1;
-        todo &= todo - 1;
-        uint32_t slot, state;
-        const uint32_t tb = t0 + b;
-        const uint32_t c = wide_expand_warp(nodes, rootmark, tb + 1u, lane, s_buf[wib], slot, state);
-        if (lane < c) {
-            ChildSlot s = nodes[slot >> 1].c[slot & 1u];
-            if (state == kItemWide) {
-                const uint32_t r = s.ref;
-                s.ref = wfirst[r - 1];
-                s.cnt = kWideFlag | wcnt[r - 1];
-            }
-            wchild[wfirst[tb] + lane] = s;
+    const uint32_t n = total ? *total : 0u;
+    for (uint32_t i = i0; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t e = wslot[i];
+        ChildSlot s = nodes[e >> 2].c[(e >> 1) & 1u];
+        if (e & 1u) {
+            const uint32_t r = s.ref;
+            s.ref = wfirst[r - 1];
+            s.cnt = kWideFlag | wcnt[r - 1];
         }
+        wchild[i] = s;
     }
 }
 
 int build_wide(uint32_t n, const Node* nodes, const uint32_t* parent, const uint32_t* rootmark, MapHeader* hdr,
                const WideBuffers& wb, cudaStream_t st) {
-    const uint32_t bound = n > 1 ? n - 1 : 1;   // internal nodes are at most n - 1
-    const uint32_t wgrid = (bound + 32u * 8u - 1u) / (32u * 8u);   // 8 warps per block, 32 nodes per warp
     if (n > 1) {
-        cudaMemsetAsync(wb.scratch, 0, wide_scan_words(n) * sizeof(uint32_t), st);
-        k_wide_count<<<wgrid, 256, 0, st>>>(nodes, parent, rootmark, hdr, bound, wb.wflag, wb.wcnt, wb.wfirst,
-                                            wb.scratch, &hdr->errors);
+        const uint32_t bound = n - 1;   // internal nodes are at most n - 1
+        cudaMemsetAsync(wb.scratch, 0, sizeof(uint32_t), st);
+        k_wide_count<<<(bound + 255u) / 256u, 256, 0, st>>>(nodes, parent, rootmark, hdr, bound, wb.wcnt, wb.wfirst,
+                                                            wb.wslot, wb.scratch);
     }
-    k_wide_emit<<<n > 1 ? wgrid : 1, 256, 0, st>>>(nodes, rootmark, wb.wflag, wb.wcnt, wb.wfirst, hdr,
-                                                  n > 1 ? bound : 0, wb.wchild, wb.wroot);
+    const uint32_t egrid = n > 1 ? std::min((n + 255u) / 256u, kWideEmitBlocks) : 1u;
+    k_wide_emit<<<egrid, 256, 0, st>>>(nodes, wb.wslot, wb.wcnt, wb.wfirst, n > 1 ? wb.scratch : nullptr, wb.wchild, wb.wroot);
     return n > 1 ? 2 : 1;
 }
 

@@ -40,68 +40,13 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
     return warp_prefix + x - v;
 }
 
-// Relaxed 64-bit loads and stores of the look-back words (status and value
-// in one word, so no other data is ordered by them).
-__device__ __forceinline__ void st_relaxed_u64(uint64_t* p, uint64_t v) {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ uint64_t ld_relaxed_u64(const uint64_t* p) {
-    uint64_t v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Polls of one look-back word before a wait gives up (sets kErrWait).
-constexpr uint32_t kLookbackWaitLimit = 1u << 22;
-
-// Decoupled look-back over one value per tile (D. Merrill and M. Garland,
-// "Single-pass Parallel Prefix Scan with Decoupled Look-back", 2016), called
-// by all 32 lanes of one warp of the block that holds tile `tile`.  The tile
-// publishes its aggregate; lane l then reads the word of tile base - l, 32
-// earlier tiles per step, waits until all 32 have published, and adds their
-// values up to the nearest one holding an inclusive prefix (or all 32
-// aggregates, then the next 32).  The tile publishes its own inclusive
-// prefix; every lane returns the exclusive prefix.  words: one uint64 per
-// tile, cleared before the launch; status in bits 62-63 (1 aggregate, 2
-// inclusive prefix).  Tiles must be taken in the order blocks start (an
-// atomic ticket), so that a tile only waits for tiles whose blocks are
-// running and publish their aggregates before they wait themselves.
-__device__ __forceinline__ uint64_t warp_lookback_exclusive(uint64_t* words, uint32_t tile, uint64_t agg,
-                                                            uint32_t* err) {
-    constexpr uint64_t kAgg = 1ull << 62, kPrefix = 2ull << 62, kValue = (1ull << 62) - 1ull;
-    const uint32_t lane = threadIdx.x & 31u;
-    if (tile == 0) {
-        if (lane == 0) st_relaxed_u64(words, kPrefix | agg);
-        return 0;
-    }
-    if (lane == 0) st_relaxed_u64(words + tile, kAgg | agg);
-    uint64_t before = 0;
-    int64_t base = (int64_t)tile - 1;
-    uint32_t polls = 0;
-    for (;;) {
-        const int64_t t = base - (int64_t)lane;
-        uint64_t w = t >= 0 ? ld_relaxed_u64(words + t) : kPrefix;   // before tile 0: a zero prefix
-        bool gave_up = false;
-        while (__any_sync(0xffffffffu, (w >> 62) == 0)) {
-            if (++polls > kLookbackWaitLimit) { gave_up = true; break; }   // never expected
-            if (polls > 32) __nanosleep(64);
-            if ((w >> 62) == 0) w = ld_relaxed_u64(words + t);
-        }
-        if (gave_up) {
-            if (lane == 0 && err) atomicOr(err, kErrWait);
-            break;
-        }
-        const uint32_t pm = __ballot_sync(0xffffffffu, (w >> 62) == 2);
-        uint64_t v = w & kValue;
-        if (pm && lane > (uint32_t)(__ffs(pm) - 1)) v = 0;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        before += v;
-        if (pm) break;
-        base -= 32;
-    }
-    if (lane == 0) st_relaxed_u64(words + tile, kPrefix | (before + agg));
-    return before;
+// One 32-byte load (sm_100: 256 bits a lane) from a 32-byte aligned address of
+// memory that no running kernel writes.  A gather's cost in L1 is the lines it
+// touches, once per load: a record read in one load instead of two pays half.
+__device__ __forceinline__ void ld_record32(const void* p, uint32_t (&v)[8]) {
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+        : "l"(p));
 }
 
 // pm_sort.cu
@@ -109,6 +54,12 @@ size_t scan_scratch_words(uint32_t n);
 int exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* scratch, uint32_t* total_out,
                    cudaStream_t st);
 size_t sort_scratch_words(uint32_t n);
+// Up to this many photons the last pass moves them.  Before it the order is by
+// the low bits only, so its reads are scattered over the whole input: above, they
+// miss L2 (20.5M photons in 64 maps: 1.37 ms for that pass, 0.16 for the others),
+// and a pass over the sorted order, whose reads are near one another, follows
+// instead.
+constexpr uint32_t kGatherInSortMax = 1u << 21;
 struct SortGather {   // the last pass moves the photons, not the values (n >= 2 only)
     const float4* in_pos;
     const float4* in_pow;
@@ -173,17 +124,16 @@ struct BuildBuffers {
 };
 
 struct WideBuffers {
-    uint32_t* wflag;       // per compacted node: is a wide node
     uint32_t* wcnt;        // per wide node: child count
-    uint32_t* wfirst;      // scan of wcnt: first child slot
+    uint32_t* wfirst;      // per wide node: first child slot
+    uint32_t* wslot;       // per child slot of a wide node: binary slot << 1 | wide
     ChildSlot* wchild;     // child slots of all wide nodes
     ChildSlot* wroot;      // start slot of the wide traversal
-    uint32_t* scratch;     // child-count scan: ticket, total, look-back words (wide_scan_words)
+    uint32_t* scratch;     // one word: child slots taken
 };
 
 // pm_build.cu
 size_t build_bytes_needed(uint32_t n);
-size_t wide_scan_words(uint32_t n);   // WideBuffers::scratch
 // Returns the number of kernels launched; sort_done (if set) is recorded on
 // the stream right after the radix sort.
 // The whole single-map build, binary and 32-wide tree.
