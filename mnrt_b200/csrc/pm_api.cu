@@ -52,7 +52,7 @@ struct pm_map {
     DevBuf stats;           // query counters (profiling level 2)
     // backward (pm_query_backward): pair sort, per-query records, segments,
     // FP64 running sums, and the forward outputs when the kNN is recomputed
-    DevBuf bvals, bvals1, bkeys0, bkeys1, bscratch, blong, qrec, seg_start, seg_end, acc;
+    DevBuf bvals, bvals1, bkeys0, bkeys1, bscratch, blong, qrec, bphoton, seg_start, seg_end, acc;
     DevBuf rnbr, rcnt, rr2, rrad;
     DevBuf gnrm, gest;        // pm_gather_for: flipped normals, estimates
     // PM_MODE_ZHOU_COMPAT: node radius estimates of the current tree, kept
@@ -148,6 +148,9 @@ pm_status buf_ensure(pm_map* m, DevBuf& b, size_t bytes, const char* name) {
 }
 
 template <class T> T* P(const DevBuf& b) { return reinterpret_cast<T*>(b.ptr); }
+template <class T> T* align32(const DevBuf& b) {
+    return reinterpret_cast<T*>((reinterpret_cast<uintptr_t>(b.ptr) + 31u) & ~(uintptr_t)31u);
+}
 
 
 // Query counts stay below 2^31: slot, round and grid arithmetic in the
@@ -332,7 +335,7 @@ pm_status pm_destroy(pm_map* m) {
                      &m->arrive, &m->nleaf, &m->partials, &m->wslot, &m->wcnt, &m->wfirst,
                      &m->wchild, &m->wroot, &m->wscan, &m->rootmark, &m->qkeys0, &m->qkeys1, &m->qvals0, &m->qvals1,
                      &m->qscratch, &m->counter, &m->fixq, &m->qsorted, &m->stats, &m->bvals, &m->bvals1, &m->bkeys0, &m->bkeys1, &m->blong,
-                     &m->bscratch, &m->qrec, &m->seg_start, &m->seg_end, &m->acc, &m->rnbr,
+                     &m->bscratch, &m->qrec, &m->bphoton, &m->seg_start, &m->seg_end, &m->acc, &m->rnbr,
                      &m->rcnt, &m->rr2, &m->rrad, &m->gnrm, &m->gest, &m->compat_est, &m->mpos, &m->mpow, &m->mflags,
                      &m->mrank, &m->mscan, &m->ic_pslot, &m->ic_level, &m->ic_range, &m->ic_center,
                      &m->ic_normal, &m->ic_est, &m->ic_exact, &m->ic_coarse, &m->ic_fin, &m->ic_work0, &m->ic_work1,
@@ -661,7 +664,9 @@ static pm_status ensure_bwd_capacity(pm_map* m, uint32_t chunk_q, uint32_t k, bo
     }
     ENSURE(bscratch, scratch_bytes);
     ENSURE(blong, ((size_t)n + 1) * sizeof(uint32_t));
-    ENSURE(qrec, qc * sizeof(BwdQuery));
+    // 32-byte loads, and a caller's allocator may align to 16 only
+    ENSURE(qrec, qc * sizeof(BwdQuery) + 32);
+    ENSURE(bphoton, (size_t)n * sizeof(BwdPhoton) + 32);
     ENSURE(seg_start, (size_t)n * sizeof(uint32_t));
     ENSURE(seg_end, (size_t)n * sizeof(uint32_t));
     if (chunked) ENSURE(acc, (size_t)n * 6 * sizeof(double));
@@ -720,7 +725,8 @@ pm_status pm_query_backward(pm_map* m, const pm_query_desc* desc, const float* d
     a.n = m->n; a.k = k; a.r_max = desc->r_max; a.filter = desc->filter;
     a.cone_k = desc->filter == PM_FILTER_CONE ? desc->cone_k : 1.0f;
     a.min_found = desc->min_found;
-    a.qrec = P<BwdQuery>(m->qrec);
+    a.qrec = align32<BwdQuery>(m->qrec);
+    a.photon = align32<BwdPhoton>(m->bphoton);
     a.vals = nullptr; a.cursor = nullptr; a.pair_cap = 0;
     a.nbr = nullptr; a.count_in = nullptr; a.order = nullptr;
     BwdBuffers b;
@@ -730,7 +736,7 @@ pm_status pm_query_backward(pm_map* m, const pm_query_desc* desc, const float* d
     b.seg_start = P<uint32_t>(m->seg_start); b.seg_end = P<uint32_t>(m->seg_end);
     b.long_count = P<uint32_t>(m->blong); b.long_list = b.long_count + 1;
     b.acc = P<double>(m->acc);
-    int nl = 0;
+    int nl = bwd_pack(a.pos, a.pow, m->n, align32<BwdPhoton>(m->bphoton), st);
     for (uint32_t c = 0; c < nchunks; ++c) {
         const uint32_t q0 = c * chunk;
         const uint32_t nqc = nq ? ((nq - q0) < chunk ? (nq - q0) : chunk) : 0;

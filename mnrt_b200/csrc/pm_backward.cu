@@ -90,7 +90,29 @@ __device__ __forceinline__ void weight_terms(int filter, double d2, double rinv,
     }
 }
 
-__device__ __forceinline__ double dist2_d(const float4& a, const float4& b) {
+__device__ __forceinline__ BwdPhoton load_photon(const BwdPhoton* p) {
+    uint32_t v[8];
+    ld_record32(p, v);
+    return BwdPhoton{__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), v[3],
+                     __uint_as_float(v[4]), __uint_as_float(v[5]), __uint_as_float(v[6]), v[7]};
+}
+
+__device__ __forceinline__ BwdQuery load_query(const BwdQuery* p) {
+    uint32_t v[8], w[8];
+    ld_record32(p, v);
+    ld_record32(reinterpret_cast<const unsigned char*>(p) + 32, w);
+    BwdQuery r;
+    r.gx = __hiloint2double((int)v[1], (int)v[0]);
+    r.gy = __hiloint2double((int)v[3], (int)v[2]);
+    r.gz = __hiloint2double((int)v[5], (int)v[4]);
+    r.G = __hiloint2double((int)v[7], (int)v[6]);
+    r.rinv = __hiloint2double((int)w[1], (int)w[0]);
+    r.qx = __uint_as_float(w[2]); r.qy = __uint_as_float(w[3]); r.qz = __uint_as_float(w[4]);
+    r.nx = __uint_as_float(w[5]); r.ny = __uint_as_float(w[6]); r.nz = __uint_as_float(w[7]);
+    return r;
+}
+
+__device__ __forceinline__ double dist2_d(const BwdPhoton& a, const float4& b) {
     const double dx = (double)a.x - (double)b.x, dy = (double)a.y - (double)b.y, dz = (double)a.z - (double)b.z;
     return dx * dx + dy * dy + dz * dz;
 }
@@ -141,16 +163,32 @@ __device__ __forceinline__ BwdHead bwd_head(const BwdArgs& a, uint32_t ql, uint3
     h.cnt = bwd_found(a, ql, lane);
     h.qp = a.qpos[q];
     h.r2 = (double)a.r_max * (double)a.r_max;
-    if (h.cnt == k) h.r2 = dist2_d(a.pos[a.inv[row[k - 1]]], h.qp);
+    if (h.cnt == k) h.r2 = dist2_d(load_photon(a.photon + row[k - 1]), h.qp);
     h.active = h.cnt > 0 && h.cnt >= a.min_found && h.r2 > 0.0 && isfinite(h.qp.x) && isfinite(h.qp.y) &&
                isfinite(h.qp.z);
     return h;
 }
 
+// Photon records in caller order, which the neighbour lists name: the
+// per-query pass then gathers one 32-byte record per pair in one load, in place
+// of the inverse permutation, the position and the flux.  A gather's cost is
+// the L1 lines it touches, once per load: 1.47 -> 1.26 ms for that pass (cold;
+// 1M x 1M, k = 64), and 0.71 -> 0.54 ms for the per-photon pass, whose 64-byte
+// query records take two such loads instead of four.
+__global__ void k_bwd_pack(const float4* __restrict__ pos, const float4* __restrict__ pw, uint32_t n,
+                           BwdPhoton* __restrict__ out) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const float4 p = pos[t], w = pw[t];
+    out[__float_as_uint(p.w)] = BwdPhoton{p.x, p.y, p.z, t, w.x, w.y, w.z, __float_as_uint(w.w)};
+}
+
 // Warp per query, in caller order: one count per placed pair on its
 // photon's cursor (the cursors are cleared before; the scan then turns the
 // counts into segment starts).  Two dependent loads per pair (row, inverse
-// permutation) and no per-query gathers: the pass is latency-bound.
+// permutation) and no per-query gathers: the pass is latency-bound.  (Keeping
+// the count's old value as the pair's slot, so that the per-query pass needs no
+// atomics, cost this pass 0.08 ms and gained that one nothing at k = 64.)
 __global__ void __launch_bounds__(256) k_bwd_count(BwdArgs a, uint32_t q0, uint32_t nq_chunk) {
     (void)q0;
     const uint32_t ql = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -201,19 +239,18 @@ __global__ void __launch_bounds__(256, 5) k_bwd_prep(BwdArgs a, uint32_t q0, uin
             a.vals[pair0 + j] = val;
             continue;
         }
-        const uint32_t p = a.inv[row[j]];
-        const uint32_t slot = kPlace ? atomicAdd(&a.cursor[p], 1u) : 0u;
-        const float4 pp = a.pos[p], pw = a.pow[p];
-        if (active && front_rn(qn.x, qn.y, qn.z, __float_as_uint(pw.w))) {
+        const BwdPhoton pp = load_photon(a.photon + row[j]);
+        const uint32_t slot = kPlace ? atomicAdd(&a.cursor[pp.tree], 1u) : 0u;
+        if (active && front_rn(qn.x, qn.y, qn.z, pp.dir)) {
             double w, dwd, dwr;
             weight_terms(a.filter, dist2_d(pp, qp), rinv, inv_r2, w, dwd, dwr);
-            S0 += w * pw.x; S1 += w * pw.y; S2 += w * pw.z;
-            T0 += dwr * pw.x; T1 += dwr * pw.y; T2 += dwr * pw.z;
+            S0 += w * pp.r; S1 += w * pp.g; S2 += w * pp.b;
+            T0 += dwr * pp.r; T1 += dwr * pp.g; T2 += dwr * pp.b;
         }
         if (kPlace) {
             if (slot < a.pair_cap) a.vals[slot] = val;
         } else {
-            a.keys[pair0 + j] = p;
+            a.keys[pair0 + j] = pp.tree;
             a.vals[pair0 + j] = val;
         }
     }
@@ -412,14 +449,14 @@ __global__ void k_bwd_reduce(BwdArgs a, uint32_t q0, const uint32_t* __restrict_
         // software pipeline: the next entry's record and the value after it
         // load while this entry's math runs (the sums keep their order)
         uint32_t vnext = sorted_vals[b];   // query << 1 | (the photon is the query's k-th)
-        BwdQuery rnext = a.qrec[vnext >> 1];
+        BwdQuery rnext = load_query(a.qrec + (vnext >> 1));
         uint32_t vafter = b + 1 < e ? sorted_vals[b + 1] : 0u;
         for (uint32_t i = b; i < e; ++i) {
             const uint32_t v = vnext;
             const BwdQuery rec = rnext;
             if (i + 1 < e) {
                 vnext = vafter;
-                rnext = a.qrec[vafter >> 1];
+                rnext = load_query(a.qrec + (vafter >> 1));
                 vafter = i + 2 < e ? sorted_vals[i + 2] : 0u;
             }
             const double rinv = rec.rinv;
@@ -458,6 +495,12 @@ size_t bwd_scratch_words(uint32_t n, uint64_t pairs, bool sort_path) {
     const size_t scan = scan_scratch_words(n) + 1;
     const size_t sort = sort_path ? sort_scratch_words((uint32_t)pairs) + 64 : 0;
     return scan > sort ? scan : sort;
+}
+
+int bwd_pack(const float4* pos, const float4* pow, uint32_t n, BwdPhoton* out, cudaStream_t st) {
+    if (!n) return 0;
+    k_bwd_pack<<<(n + 255) / 256, 256, 0, st>>>(pos, pow, n, out);
+    return 1;
 }
 
 int backward_chunk(const BwdArgs& a, uint32_t q0, uint32_t nq_chunk, bool first, bool last, const BwdBuffers& b,

@@ -254,7 +254,7 @@ int scale_rgb(float4* pw, uint32_t n, float scale, cudaStream_t st);
 // pm_backward.cu
 // Per-query record of the adjoint, 64 bytes: everything the per-photon pass
 // needs about one query in one aligned load.
-struct __align__(16) BwdQuery {
+struct __align__(32) BwdQuery {
     double gx, gy, gz;        // dL/dE * norm per channel
     double G;                 // the k-th neighbour's r^2 path (0 unless k were found)
     double rinv;              // the filter's reciprocal: 1 / (k_c r) cone, 1 / r^2 Epanechnikov, 1 box;
@@ -264,7 +264,18 @@ struct __align__(16) BwdQuery {
 };
 static_assert(sizeof(BwdQuery) == 64, "one 64-byte record per query");
 
+// A photon as the adjoint's per-query pass gathers it, in caller order (the
+// order the neighbour lists name): one aligned 32-byte load gives all of it.
+struct __align__(32) BwdPhoton {
+    float x, y, z;
+    uint32_t tree;            // tree position
+    float r, g, b;
+    uint32_t dir;
+};
+static_assert(sizeof(BwdPhoton) == 32, "one 32-byte record per photon");
+
 struct BwdArgs {
+    const BwdPhoton* photon;  // caller order (bwd_pack)
     const float4* pos;        // tree order
     const float4* pow;
     const uint32_t* inv;      // caller index -> tree position
@@ -300,6 +311,7 @@ struct BwdBuffers {
 constexpr uint64_t kBwdPlaceMaxFanIn = 256;
 inline bool bwd_sort_path(uint64_t pairs, uint32_t n) { return pairs > kBwdPlaceMaxFanIn * (uint64_t)n; }
 size_t bwd_scratch_words(uint32_t n, uint64_t pairs, bool sort_path);
+int bwd_pack(const float4* pos, const float4* pow, uint32_t n, BwdPhoton* out, cudaStream_t st);
 int backward_chunk(const BwdArgs& a, uint32_t q0, uint32_t nq_chunk, bool first, bool last, const BwdBuffers& b,
                    float4* grad_pow, float4* grad_pos, cudaStream_t st);
 
