@@ -447,9 +447,10 @@ static pm_status compat_run(pm_map* m, const pm_query_desc* desc, const float* d
     const uint32_t max_slots = 2 * (m->cap_photons + 1);
     if (m->compat_gen != m->build_gen || m->compat_k != desc->k || m->compat_r != desc->r_max ||
         m->compat_iters != iters) {
-        if (m->compat_est.bytes < (size_t)max_slots * sizeof(float)) {
+        const size_t bytes = ((size_t)max_slots + 1) * sizeof(float);   // and the kernel's work counter
+        if (m->compat_est.bytes < bytes) {
             if (capturing(st)) return fail(m, PM_ERR_STATE, "compat storage must grow during stream capture");
-            pm_status s = buf_ensure(m, m->compat_est, (size_t)max_slots * sizeof(float), "compat node estimates");
+            pm_status s = buf_ensure(m, m->compat_est, bytes, "compat node estimates");
             if (s != PM_OK) return s;
         }
         m->launches += (uint64_t)compat_node_estimates(view_of(m), max_slots, desc->r_max, desc->k, iters,

@@ -198,18 +198,22 @@ __device__ float refine_radius(const MapView& m, float qx, float qy, float qz, f
     return r_max;
 }
 
-// One warp per slot, grid-stride; the slot count comes from the map header (2
-// per internal node plus the super-root's two).
+// One warp per slot, taken from a counter (a slot in a dense blob walks a
+// hundred nodes more than one beside it); the slot count comes from the map
+// header (2 per internal node plus the super-root's two).
 __global__ void __launch_bounds__(32 * kCompatWarps) k_compat_nodes(MapView m, uint32_t max_slots, float rmax, uint32_t k,
-                                                                    uint32_t iters, float* est) {
+                                                                    uint32_t iters, float* est, uint32_t* next) {
     __shared__ CompatSmem s_warp[kCompatWarps];
     const uint32_t lane = lane_id();
     CompatSmem& s = s_warp[threadIdx.x >> 5];
     const uint32_t internal = m.hdr->num_nodes;
     const uint32_t nslots = min(2u * (internal + 1u), max_slots);
     const bool enabled = 2 * internal + 1 >= 1000;   // node estimates are skipped for small trees
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t sid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; sid < nslots; sid += warps) {
+    for (;;) {
+        uint32_t sid = 0;
+        if (lane == 0) sid = atomicAdd(next, 1u);
+        sid = __shfl_sync(kFull, sid, 0);
+        if (sid >= nslots) break;
         float e = INFINITY;
         float lo[3], hi[3];
         uint32_t ref, cnt;
@@ -274,7 +278,7 @@ struct CompatArgs {
     uint32_t* out_count;
 };
 
-__global__ void __launch_bounds__(32 * kCompatWarps) k_compat_query(CompatArgs a) {
+__global__ void __launch_bounds__(32 * kCompatWarps, 4) k_compat_query(CompatArgs a) {
     __shared__ CompatSmem s_warp[kCompatWarps];
     const uint32_t lane = lane_id(), lt = (1u << lane) - 1u;
     CompatSmem& s = s_warp[threadIdx.x >> 5];
@@ -381,11 +385,13 @@ int sm_count() {
 
 }  // namespace
 
-// est holds max_slots floats; max_slots >= 2 * (internal nodes + 1).
+// est holds max_slots floats, max_slots >= 2 * (internal nodes + 1), and one word more.
 int compat_node_estimates(const MapView& m, uint32_t max_slots, float rmax, uint32_t k, uint32_t iters, float* est,
                           cudaStream_t st) {
-    const uint32_t need = (max_slots + kCompatWarps - 1) / kCompatWarps, most = (uint32_t)sm_count() * 8u;
-    k_compat_nodes<<<need < most ? need : most, 32 * kCompatWarps, 0, st>>>(m, max_slots, rmax, k, iters, est);
+    const uint32_t need = (max_slots + kCompatWarps - 1) / kCompatWarps, most = (uint32_t)sm_count() * 4u;
+    uint32_t* next = reinterpret_cast<uint32_t*>(est + max_slots);
+    cudaMemsetAsync(next, 0, sizeof(uint32_t), st);
+    k_compat_nodes<<<need < most ? need : most, 32 * kCompatWarps, 0, st>>>(m, max_slots, rmax, k, iters, est, next);
     return 1;
 }
 
