@@ -280,15 +280,13 @@ QueryParams params_of(const pm_query_desc* d) {
     return p;
 }
 
-// Hilbert order of the queries (returns the permutation or nullptr).
+// Hilbert (or Morton) order of the queries; with qnrm also their records in it (m->qsorted).
 const uint32_t* sort_queries(pm_map* m, const float4* qpos, uint32_t nq, cudaStream_t st, int* launches,
-                             bool hilbert = true) {
-    *launches += query_order_keys(qpos, nq, P<MapHeader>(m->hdr), P<uint32_t>(m->qkeys0), P<uint32_t>(m->qvals0), st,
-                                  hilbert);
-    uint32_t* keys[2] = {P<uint32_t>(m->qkeys0), P<uint32_t>(m->qkeys1)};
-    uint32_t* vals[2] = {P<uint32_t>(m->qvals0), P<uint32_t>(m->qvals1)};
-    const int cur = radix_sort_pairs32(keys, vals, nq, kQueryKeyBits, P<uint32_t>(m->qscratch), st, launches);
-    return vals[cur];
+                             bool hilbert = true, const float4* qnrm = nullptr) {
+    uint32_t* const keys[2] = {P<uint32_t>(m->qkeys0), P<uint32_t>(m->qkeys1)};
+    uint32_t* const vals[2] = {P<uint32_t>(m->qvals0), P<uint32_t>(m->qvals1)};
+    return query_order(qpos, nq, P<MapHeader>(m->hdr), keys, vals, P<uint32_t>(m->qscratch), st, launches, hilbert, qnrm,
+                       qnrm ? P<float4>(m->qsorted) : nullptr);
 }
 
 }  // namespace
@@ -478,21 +476,25 @@ static pm_status query_exact_run(pm_map* m, const pm_query_desc* desc, const flo
     const bool prof = m->profiling && !capturing(st);
     if (prof) cudaEventRecord(m->ev[3], st);
     int nl = 0;
-    const uint32_t* order = desc->order == PM_ORDER_SORTED ? sort_queries(m, qpos, nq, st, &nl) : nullptr;
+    // the wide layout reads the 32-byte query records in processing order, so the
+    // search reads them sequentially instead of through the permutation; where the
+    // normals are still on their way the records follow the sort, which only
+    // needs the positions (6.97 -> 6.90 ms for the plain workload's search, the
+    // record pass included)
+    QueryTuning t = tuning_of(m);
+    const float4* qnrm = reinterpret_cast<const float4*>(d_qnrm4);
+    const bool recs = t.layout == 2;
+    const uint32_t* order = desc->order == PM_ORDER_SORTED
+                                ? sort_queries(m, qpos, nq, st, &nl, true, recs && !nrm_ready ? qnrm : nullptr) : nullptr;
     if (prof) cudaEventRecord(m->ev[4], st);
     if (nrm_ready) cudaStreamWaitEvent(st, nrm_ready, 0);
     QueryOutputs out{reinterpret_cast<float4*>(d_rad4), d_nbr, d_r2, d_count};
-    QueryTuning t = tuning_of(m);
-    if (order && t.layout == 2) {
-        // the 32-byte query records in processing order, so the search reads them
-        // sequentially instead of through the permutation (after the normals have
-        // arrived: the sort above only needs the positions); 6.97 -> 6.90 ms for
-        // the plain workload's search, this launch included
-        nl += gather_queries(order, qpos, reinterpret_cast<const float4*>(d_qnrm4), nq, P<float4>(m->qsorted), st);
+    if (order && recs) {
+        if (nrm_ready) nl += gather_queries(order, qpos, qnrm, nq, P<float4>(m->qsorted), st);
         t.qsorted = P<float4>(m->qsorted);
     }
     nl += query_knn(view_of(m), params_of(desc), qpos, reinterpret_cast<const float4*>(d_qnrm4), order, nq, out,
-                    P<uint32_t>(m->counter), P<uint32_t>(m->fixq), t, st);
+                    P<uint32_t>(m->counter), P<uint32_t>(m->fixq), P<float>(m->qkeys0), t, st);
     if (prof) cudaEventRecord(m->ev[5], st);
     m->have_query_ev = prof;
     m->query_launches = (uint32_t)nl;
@@ -743,14 +745,16 @@ pm_status pm_query_backward(pm_map* m, const pm_query_desc* desc, const float* d
         const uint32_t nqc = nq ? ((nq - q0) < chunk ? (nq - q0) : chunk) : 0;
         // the chunk's queries in Hilbert order: the recomputed forward and the
         // adjoint's per-query pass walk them in it
-        a.order = (sorted && nqc > 0) ? sort_queries(m, a.qpos + q0, nqc, st, &nl) : nullptr;
+        a.order = (sorted && nqc > 0) ? sort_queries(m, a.qpos + q0, nqc, st, &nl, true, recompute && m->kbuf_layout == PM_KBUF_WIDE ? a.qnrm + q0 : nullptr)
+                                        : nullptr;
         if (recompute) {
             if (nqc > 0) {
                 QueryOutputs out{P<float4>(m->rrad), P<uint32_t>(m->rnbr), P<float>(m->rr2), P<uint32_t>(m->rcnt)};
                 QueryTuning t = tuning_of(m);
                 t.stats = nullptr;
+                if (a.order && t.layout == PM_KBUF_WIDE) t.qsorted = P<float4>(m->qsorted);
                 nl += query_knn(view_of(m), params_of(desc), a.qpos + q0, a.qnrm + q0, a.order, nqc, out,
-                                P<uint32_t>(m->counter), P<uint32_t>(m->fixq), t, st);
+                                P<uint32_t>(m->counter), P<uint32_t>(m->fixq), P<float>(m->qkeys0), t, st);
             }
             a.nbr = P<uint32_t>(m->rnbr);
             a.count_in = P<uint32_t>(m->rcnt);
@@ -807,14 +811,17 @@ pm_status pm_gather_for(pm_map* m, const pm_query_desc* desc, const float* d_hit
     } else {
         nl += gather_normals(reinterpret_cast<const float4*>(d_hit_nrm4), reinterpret_cast<const float4*>(d_ray_dir4), n,
                              P<float4>(m->gnrm), st);
-        const uint32_t* order = desc->order == PM_ORDER_SORTED ? sort_queries(m, hit, n, st, &nl) : nullptr;
+        const bool recs = m->kbuf_layout == PM_KBUF_WIDE;   // query records in processing order
+        const uint32_t* order = desc->order == PM_ORDER_SORTED
+                                    ? sort_queries(m, hit, n, st, &nl, true, recs ? P<float4>(m->gnrm) : nullptr) : nullptr;
         QueryParams qp = params_of(desc);
         if (!d_clr_diffuse4) qp.min_found = 0;   // photon visualisation keeps every estimate (GPU/photon_knn.cu:515-519)
         QueryOutputs out{P<float4>(m->gest), nullptr, nullptr, nullptr};
         QueryTuning t = tuning_of(m);
         t.stats = nullptr;
+        if (order && recs) t.qsorted = P<float4>(m->qsorted);
         nl += query_knn(view_of(m), qp, hit, P<float4>(m->gnrm), order, n, out, P<uint32_t>(m->counter),
-                        P<uint32_t>(m->fixq), t, st);
+                        P<uint32_t>(m->fixq), P<float>(m->qkeys0), t, st);
     }
     nl += gather_accumulate(P<float4>(m->gest), hit, reinterpret_cast<const float4*>(d_ray_origin4),
                             reinterpret_cast<const float4*>(d_ray_influence4),
@@ -912,12 +919,15 @@ pm_status pm_icut_build(pm_map* m, const pm_icut_desc* cut, const pm_query_desc*
     } else {
         s = ensure_query_capacity(m, ns, st);
         if (s != PM_OK) return s;
-        const uint32_t* order = node_query->order == PM_ORDER_SORTED ? sort_queries(m, b.center, ns, st, &nl) : nullptr;
+        const bool recs = m->kbuf_layout == PM_KBUF_WIDE;   // query records in processing order
+        const uint32_t* order = node_query->order == PM_ORDER_SORTED
+                                    ? sort_queries(m, b.center, ns, st, &nl, true, recs ? b.normal : nullptr) : nullptr;
         QueryOutputs out{b.exact, nullptr, nullptr, nullptr};
         QueryTuning t = tuning_of(m);
         t.stats = nullptr;
+        if (order && recs) t.qsorted = P<float4>(m->qsorted);
         nl += query_knn(v, params_of(node_query), b.center, b.normal, order, ns, out, P<uint32_t>(m->counter),
-                        P<uint32_t>(m->fixq), t, st);
+                        P<uint32_t>(m->fixq), P<float>(m->qkeys0), t, st);
     }
     nl += icut_final(v, ns, p, b, st);
     m->launches += (uint64_t)nl;
@@ -1213,17 +1223,15 @@ extern "C" pm_status pm_query_noalloc(pm_map* m, const pm_query_desc* desc, cons
                              reinterpret_cast<uint32_t*>(base + kNoallocKeys1)};
         uint32_t* vals[2] = {reinterpret_cast<uint32_t*>(base + kNoallocVals0),
                              reinterpret_cast<uint32_t*>(base + kNoallocVals1)};
-        nl += query_order_keys(qpos, nq, P<MapHeader>(m->hdr), keys[0], vals[0], st);
-        const int cur = radix_sort_pairs32(keys, vals, nq, kQueryKeyBits, reinterpret_cast<uint32_t*>(base + kNoallocSort),
-                                           st, &nl);
-        order = vals[cur];
+        order = query_order(qpos, nq, P<MapHeader>(m->hdr), keys, vals, reinterpret_cast<uint32_t*>(base + kNoallocSort),
+                            st, &nl, true);
     }
     QueryTuning t = tuning_of(m);
     t.stats = nullptr;
     QueryOutputs out{reinterpret_cast<float4*>(d_rad4), d_nbr, d_r2, d_count};
     nl += query_knn(view_of(m), params_of(desc), qpos, reinterpret_cast<const float4*>(d_qnrm4), order, nq, out,
                     reinterpret_cast<uint32_t*>(base + kNoallocCounter), reinterpret_cast<uint32_t*>(base + kNoallocFix),
-                    t, st);
+                    reinterpret_cast<float*>(base + kNoallocKeys0), t, st);
     // no phase events and no traversal counters here: pm_last_timings then
     // reports this call's launch count and no query times
     m->have_query_ev = false;
@@ -1359,7 +1367,7 @@ pm_status batch_build_device(pm_batch* b, const float* d_pos4, const float* d_po
     return check_cuda(m, "pm_batch_build");
 }
 
-pm_status batch_query_device(pm_batch* b, uint32_t kmax, const float* d_qpos4, const float* d_qnrm4, uint32_t nq,
+pm_status batch_query_device(pm_batch* b, uint32_t kmax, uint64_t pairs, const float* d_qpos4, const float* d_qnrm4, uint32_t nq,
                              float* d_rad4, uint32_t* d_nbr, float* d_r2, uint32_t* d_count, cudaStream_t st) {
     pm_map* m = b->m;
     if (nq == 0) return PM_OK;
@@ -1374,9 +1382,15 @@ pm_status batch_query_device(pm_batch* b, uint32_t kmax, const float* d_qpos4, c
     QueryOutputs out{reinterpret_cast<float4*>(d_rad4), d_nbr, d_r2, d_count};
     QueryTuning t = tuning_of(m);
     t.stats = nullptr;
-    nl += query_knn_batch(view_of(m), P<BatchQuery>(b->bq), P<BatchGeom>(b->geom), kmax, qpos,
+    if (t.layout == PM_KBUF_WIDE) {   // query records in processing order
+        nl += gather_queries(vals[cur], qpos, reinterpret_cast<const float4*>(d_qnrm4), nq, P<float4>(m->qsorted), st);
+        t.qsorted = P<float4>(m->qsorted);
+    }
+    MapView v = view_of(m);
+    v.n = b->total_photons;
+    nl += query_knn_batch(v, P<BatchQuery>(b->bq), P<BatchGeom>(b->geom), kmax, pairs, qpos,
                           reinterpret_cast<const float4*>(d_qnrm4), vals[cur], keys[cur], nq, out, P<uint32_t>(m->counter),
-                          P<uint32_t>(m->fixq), t, st);
+                          P<uint32_t>(m->fixq), reinterpret_cast<float*>(keys[cur ^ 1]), t, st);
     m->launches += (uint64_t)nl;
     b->query_launches = (uint32_t)nl;
     return check_cuda(m, "pm_batch_query");
@@ -1473,7 +1487,7 @@ pm_status pm_batch_query(pm_batch* b, const pm_query_desc* descs, const float* d
     if (s != PM_OK) return s;
     if ((s = ensure_query_capacity(b->m, nq, st)) != PM_OK) return s;
     if ((s = batch_upload_queries(b, descs, query_offsets, &kmax, &nbr_total)) != PM_OK) return s;
-    return batch_query_device(b, kmax, d_qpos4, d_qnrm4, nq, d_rad4, d_nbr, d_r2, d_count, st);
+    return batch_query_device(b, kmax, nbr_total, d_qpos4, d_qnrm4, nq, d_rad4, d_nbr, d_r2, d_count, st);
 }
 
 pm_status pm_batch_capture(pm_batch* b, const float* d_pos4, const float* d_pow4, const uint32_t* photon_offsets,
@@ -1497,7 +1511,7 @@ pm_status pm_batch_capture(pm_batch* b, const float* d_pos4, const float* d_pow4
     if (cudaStreamBeginCapture(b->cap_stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
         return check_cuda(b->m, "pm_batch_capture: begin");
     pm_status sb = batch_build_device(b, d_pos4, d_pow4, format, b->cap_stream);
-    pm_status sq = sb == PM_OK ? batch_query_device(b, kmax, d_qpos4, d_qnrm4, nq, d_rad4, d_nbr, d_r2, d_count,
+    pm_status sq = sb == PM_OK ? batch_query_device(b, kmax, nbr_total, d_qpos4, d_qnrm4, nq, d_rad4, d_nbr, d_r2, d_count,
                                                     b->cap_stream)
                                : sb;
     cudaGraph_t g = nullptr;

@@ -165,8 +165,12 @@ struct QueryOutputs {
     uint32_t* count;     // optional
 };
 
-int query_order_keys(const float4* qpos, uint32_t nq, const MapHeader* hdr, uint32_t* keys, uint32_t* vals,
-                       cudaStream_t st, bool hilbert = true);
+// Processing order of the queries (Hilbert, or Morton); with recs also their
+// records in that order (needs the normals).  keys and vals: two buffers of nq
+// words each, scratch: sort_scratch_words(nq).
+const uint32_t* query_order(const float4* qpos, uint32_t nq, const MapHeader* hdr, uint32_t* const keys[2],
+                            uint32_t* const vals[2], uint32_t* scratch, cudaStream_t st, int* launches, bool hilbert,
+                            const float4* qnrm = nullptr, float4* recs = nullptr);
 constexpr int kQueryKeyBits = 30;         // bits of the query Hilbert keys (sorted as uint32)
 constexpr int kBatchQueryMapShift = 30;   // batch query keys: (map id << 30) | 30-bit Hilbert index in the map's cell
 struct QueryTuning {
@@ -179,16 +183,16 @@ struct QueryTuning {
 };
 int gather_queries(const uint32_t* order, const float4* qpos, const float4* qnrm, uint32_t nq, float4* out, cudaStream_t st);
 int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const float4* qnrm,
-              const uint32_t* order, uint32_t nq, const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list,
+              const uint32_t* order, uint32_t nq, const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list, float* fix_bound,
               const QueryTuning& t, cudaStream_t st);
 int query_bruteforce(const MapView& m, const QueryParams& p, const float4* qpos, const float4* qnrm,
                       uint32_t nq, const QueryOutputs& out, cudaStream_t st);
 int query_smem_bytes_per_warp(uint32_t k);
 double filter_norm_const(int filter, float cone_k);
 
-int query_knn_batch(const MapView& m, const BatchQuery* bq, const BatchGeom* bg, uint32_t kmax, const float4* qpos,
+int query_knn_batch(const MapView& m, const BatchQuery* bq, const BatchGeom* bg, uint32_t kmax, uint64_t pairs, const float4* qpos,
                     const float4* qnrm, const uint32_t* order, const uint64_t* qkeys, uint32_t nq,
-                    const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list, const QueryTuning& t,
+                    const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list, float* fix_bound, const QueryTuning& t,
                     cudaStream_t st);
 
 // pm_batch.cu

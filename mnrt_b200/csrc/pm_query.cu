@@ -27,6 +27,8 @@
 //     the order in which neighbours were found, and every layout gives the
 //     same bits.
 #include "pm_internal.h"
+#include "pm_sort_small.cuh"
+#include <algorithm>
 
 namespace pm {
 
@@ -52,7 +54,8 @@ struct KnnArgs {
     float* out_r2;
     uint32_t* out_count;
     uint32_t* work_counter;
-    uint32_t* fix_list;       // group kernel: sorted slots of queries whose estimate needs FP64 distances
+    uint32_t* fix_list;       // sorted slots of the queries left to the fix pass (FP64 distances)
+    float* fix_bound;         // a bound of each listed query's search (exclusive, on d^2)
     const uint32_t* fix_in;   // fix pass: the list it works through
     uint32_t* fix_count;
     const uint32_t* nq_dev;   // fix pass: query count read on the device
@@ -74,6 +77,15 @@ struct KnnArgs {
     const ChildSlot* s_top;   // staged root children (shared memory) or nullptr
     uint32_t top_first;       // wchild index of the staged children
 };
+
+// Leaves the query at sorted slot `slot` to the fix pass.  The k-th neighbour is
+// known to lie below `bound`, or R^2 is given: with it the pass visits little
+// more than the answer (a handful of queries of the small configuration: 31 -> 18 us).
+__device__ __forceinline__ void fix_push(const KnnArgs& a, uint32_t slot, float bound) {
+    const uint32_t i = atomicAdd(a.fix_count, 1u);
+    a.fix_list[i] = slot;
+    a.fix_bound[i] = bound;
+}
 
 // Counters of the group kernel, accumulated when KnnArgs::stats is set.
 enum { kStatQueries = 0, kStatNodes, kStatLeaves, kStatPhotons, kStatCandidates, kStatSelections, kStatRedo,
@@ -936,7 +948,7 @@ __device__ float group_finish(const KnnArgs& a, uint64_t* buf, uint32_t& n, uint
             if (kFix) {
                 r2d = est_fp64_group<G>(a, buf, n, s, gmask, qx, qy, qz, nx, ny, nz, acc);
             } else if (s == 0) {   // re-evaluated by the fix pass (the FP32 result written below is replaced)
-                a.fix_list[atomicAdd(a.fix_count, 1u)] = slot;
+                fix_push(a, slot, n == k ? __uint_as_float(__float_as_uint(r2) + 1u) : a.r2max);
             }
         }
         rad = est_result(acc, r2d, scale, n, a.norm_c);
@@ -1108,6 +1120,11 @@ __device__ __forceinline__ void wide_traverse(const KnnArgs& a, float qx, float 
     }
 }
 
+// Candidate buffer entries per query: k rounded up to a warp, plus 96 of
+// headroom before a selection must make room (with leaves of up to 64
+// photons, 96 measured 5.90 -> 5.87 ms against 64 on the plain workload).
+__host__ __device__ inline uint32_t group_capacity(uint32_t k) { return ((k + 31u) & ~31u) + 96u; }
+
 // The wide instances are held to 64 registers (4 blocks of 256 per SM, 32
 // warps): measured fastest.  Without a bound ptxas holds them to 48
 // registers and spills; with 3 blocks (80 registers, no spills, 24 warps) the
@@ -1196,6 +1213,7 @@ __global__ void __launch_bounds__(256, kWide ? 4 : 0) k_knn_group(KnnArgs a0) {
             }
             // radius bound from the previous round's queries of this warp
             float tau0 = r2max;
+            if (kFix && inrange) tau0 = fminf(r2max, a.fix_bound[slot_q]);
 #pragma unroll
             for (int h = 0; h < QW; ++h) {
                 // one query per warp: every lane already holds its predecessor's values
@@ -1354,6 +1372,7 @@ __global__ void __launch_bounds__(256, kWide ? 4 : 0) k_knn_group(KnnArgs a0) {
     }
 }
 
+
 // Brute force: thread per query, every photon staged through shared memory.
 constexpr int kBruteThreads = 64;
 constexpr int kBruteTile = 512;
@@ -1459,12 +1478,69 @@ __global__ void k_query_order(const float4* __restrict__ qpos, uint32_t nq, cons
 // 30-bit query keys (Hilbert, or Morton when hilbert is false): 4 radix
 // passes instead of the tree's 6 (a cell is 1/1024 of the map's extent per
 // axis, finer than the query spacing of the measured workloads).
-int query_order_keys(const float4* qpos, uint32_t nq, const MapHeader* hdr, uint32_t* keys, uint32_t* vals,
-                     cudaStream_t st, bool hilbert) {
+static int query_order_keys(const float4* qpos, uint32_t nq, const MapHeader* hdr, uint32_t* keys, uint32_t* vals,
+                            cudaStream_t st, bool hilbert) {
     if (!nq) return 0;
     if (hilbert) k_query_order<true><<<(nq + 255) / 256, 256, 0, st>>>(qpos, nq, hdr, keys, vals);
     else k_query_order<false><<<(nq + 255) / 256, 256, 0, st>>>(qpos, nq, hdr, keys, vals);
     return 1;
+}
+
+// Keys and sort of up to kSmallSortMax queries in one launch: the processing
+// order, and (recs set) the query records laid out in it.
+template <bool kHilbert, int R>
+__global__ void __launch_bounds__(kSmallSortThreads, 1) k_small_query_sort(const float4* __restrict__ qpos,
+                                                                           const float4* __restrict__ qnrm, uint32_t nq,
+                                                                           const MapHeader* __restrict__ hdr,
+                                                                           uint32_t* __restrict__ order,
+                                                                           float4* __restrict__ recs) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const float ext = fmaxf(fmaxf(__fsub_rn(hdr->hi[0], hdr->lo[0]), __fsub_rn(hdr->hi[1], hdr->lo[1])),
+                            __fsub_rn(hdr->hi[2], hdr->lo[2]));
+    const float scale = (ext > 0.0f && isfinite(ext)) ? __fdiv_rn(65536.0f, ext) : 0.0f;
+    const uint32_t first = blockIdx.x * (uint32_t)(kSmallSortThreads * R) + (threadIdx.x >> 5) * 32u * R + (threadIdx.x & 31u);
+    uint32_t key[R], val[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t i = first + 32u * r;
+        const float4 p = i < nq ? qpos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        key[r] = kHilbert ? hilbert30(p.x, p.y, p.z, hdr->lo, scale) : morton30(p.x, p.y, p.z, hdr->lo, scale);
+        val[r] = i;
+    }
+    small_sort<uint32_t, R>(key, val, nq, kQueryKeyBits, smem, [&](uint32_t dst, uint32_t, uint32_t src) {
+        order[dst] = src;
+        if (recs) {
+            float4 p = qpos[src];
+            p.w = __uint_as_float(src);
+            recs[2 * (size_t)dst] = p;
+            recs[2 * (size_t)dst + 1] = qnrm[src];
+        }
+    });
+}
+
+template <bool kHilbert>
+static void small_query_sort(const float4* qpos, const float4* qnrm, uint32_t nq, const MapHeader* hdr, uint32_t* order,
+                             float4* recs, cudaStream_t st) {
+    if (nq <= kSmallSortMax / 4) launch_small_sort<uint32_t, 1>(k_small_query_sort<kHilbert, 1>, nq, st, qpos, qnrm, nq, hdr, order, recs);
+    else if (nq <= kSmallSortMax / 2) launch_small_sort<uint32_t, 2>(k_small_query_sort<kHilbert, 2>, nq, st, qpos, qnrm, nq, hdr, order, recs);
+    else launch_small_sort<uint32_t, 4>(k_small_query_sort<kHilbert, 4>, nq, st, qpos, qnrm, nq, hdr, order, recs);
+}
+
+const uint32_t* query_order(const float4* qpos, uint32_t nq, const MapHeader* hdr, uint32_t* const keys[2],
+                            uint32_t* const vals[2], uint32_t* scratch, cudaStream_t st, int* launches, bool hilbert,
+                            const float4* qnrm, float4* recs) {
+    if (nq > 1 && nq <= kSmallSortMax) {
+        if (hilbert) small_query_sort<true>(qpos, qnrm, nq, hdr, vals[0], recs, st);
+        else small_query_sort<false>(qpos, qnrm, nq, hdr, vals[0], recs, st);
+        ++*launches;
+        return vals[0];
+    }
+    *launches += query_order_keys(qpos, nq, hdr, keys[0], vals[0], st, hilbert);
+    uint32_t* k[2] = {keys[0], keys[1]};
+    uint32_t* v[2] = {vals[0], vals[1]};
+    const int cur = radix_sort_pairs32(k, v, nq, kQueryKeyBits, scratch, st, launches);
+    if (recs) *launches += gather_queries(v[cur], qpos, qnrm, nq, recs, st);
+    return v[cur];
 }
 
 int query_smem_bytes_per_warp(uint32_t k) {
@@ -1488,7 +1564,7 @@ static KnnArgs make_args(const MapView& m, const QueryParams& p, const float4* q
     a.k = p.k; a.r2max = p.r2; a.rmax = p.r; a.filter = p.filter; a.cone_k = p.cone_k; a.min_found = p.min_found;
     a.out_rad = out.rad; a.out_nbr = out.nbr; a.out_r2 = out.r2; a.out_count = out.count;
     a.work_counter = nullptr; a.rounds_per_chunk = 1;
-    a.fix_list = nullptr; a.fix_count = nullptr; a.nq_dev = nullptr; a.fix_in = nullptr;
+    a.fix_list = nullptr; a.fix_bound = nullptr; a.fix_count = nullptr; a.nq_dev = nullptr; a.fix_in = nullptr;
     a.scale_ptr = &m.hdr->fix_scale;
     a.root = &m.nodes[0].c[0];
     a.wchild = m.wchild;
@@ -1501,11 +1577,6 @@ static KnnArgs make_args(const MapView& m, const QueryParams& p, const float4* q
     return a;
 }
 
-// Candidate buffer entries per query: k rounded up to a warp, plus 96 of
-// headroom before a selection must make room (with leaves of up to 64
-// photons, 96 measured 5.90 -> 5.87 ms against 64 on the plain workload).
-uint32_t group_capacity(uint32_t k) { return ((k + 31u) & ~31u) + 96u; }
-
 int wide_smem_bytes_per_warp(uint32_t k) {
     return (int)(group_capacity(k) * sizeof(uint64_t) + 256 * sizeof(uint32_t)) + 2 * kWideStack * (int)sizeof(uint32_t);
 }
@@ -1516,20 +1587,32 @@ int group_smem_bytes_per_warp(uint32_t k, int qpw) {
 }
 
 template <class K>
-static uint32_t grid_for(K kernel, int threads, int smem, uint32_t work_items, int warps_per_block) {
+static uint32_t grid_full(K kernel, int threads, int smem) {
     if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-    if (per_sm < 1) per_sm = 1;
-    uint32_t grid = (uint32_t)(sms * per_sm);
-    const uint32_t need = (work_items + warps_per_block - 1) / warps_per_block;
-    return grid > need ? need : (grid ? grid : 1);
+    return (uint32_t)(sms * (per_sm < 1 ? 1 : per_sm));
+}
+
+// Grid for `rounds` rounds of work in chunks of at least chunk rounds.  Where
+// that many chunks would leave warps of the full grid without one, chunk is
+// lowered: a launch this small is bound by its longest warp, and a query
+// without its predecessor's radius bound costs less than waiting for it (4,095
+// queries, 1M photons, k = 100: 183 -> 58 us).
+template <class K>
+static uint32_t grid_for(K kernel, int threads, int smem, uint32_t rounds, int warps_per_block, uint32_t& chunk) {
+    const uint32_t full = grid_full(kernel, threads, smem);
+    const uint32_t fair = rounds / (full * (uint32_t)warps_per_block);
+    if (chunk > fair) chunk = fair > 1 ? fair : 1;
+    const uint32_t chunks = (rounds + chunk - 1) / chunk;
+    const uint32_t need = (chunks + warps_per_block - 1) / warps_per_block;
+    return full > need ? need : full;
 }
 
 int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const float4* qnrm,
-              const uint32_t* order, uint32_t nq, const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list,
+              const uint32_t* order, uint32_t nq, const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list, float* fix_bound,
               const QueryTuning& t, cudaStream_t st) {
     if (!nq) return 0;
     KnnArgs a = make_args(m, p, qpos, qnrm, order, nq, out);
@@ -1541,28 +1624,28 @@ int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const 
     cudaMemsetAsync(work_counter, 0, 3 * sizeof(uint32_t), st);   // work, fix count, fix work
     if (t.layout == 0) {   // one lane per query, shared-memory heap
         const int smem = query_smem_bytes_per_warp(p.k) * t.warps_per_block;
-        const uint32_t nchunks = (nq + 32u * a.rounds_per_chunk - 1) / (32u * a.rounds_per_chunk);
-        const uint32_t grid = grid_for(k_knn_tree, threads, smem, nchunks, t.warps_per_block);
+        const uint32_t grid = grid_for(k_knn_tree, threads, smem, (nq + 31u) / 32u, t.warps_per_block, a.rounds_per_chunk);
         k_knn_tree<<<grid, threads, smem, st>>>(a);
         return 1;
     }
-    if (t.layout == 2) {   // one query per warp over the 32-wide tree
+    if (t.layout == 2) {   // over the 32-wide tree
         a.qsorted = t.qsorted;
         a.cap = group_capacity(p.k);
         a.smem_per_warp = (uint32_t)wide_smem_bytes_per_warp(p.k);
         a.root = m.wroot;
         a.fix_list = fix_list;
+        a.fix_bound = fix_bound;
         a.fix_count = work_counter + 1;
         const int smem = (int)a.smem_per_warp * t.warps_per_block + kTopBytes;
-        const uint32_t nchunks = (nq + a.rounds_per_chunk - 1) / a.rounds_per_chunk;
         KnnArgs fx = a;
         fx.fix_in = fix_list;
         fx.nq_dev = work_counter + 1;
         fx.work_counter = work_counter + 2;
+        fx.rounds_per_chunk = 1;
         fx.qsorted = nullptr;
-        const uint32_t grid = grid_for(k_knn_group<32, false, false, true>, threads, smem, nchunks, t.warps_per_block);
+        const uint32_t grid = grid_for(k_knn_group<32, false, false, true>, threads, smem, nq, t.warps_per_block, a.rounds_per_chunk);
         k_knn_group<32, false, false, true><<<grid, threads, smem, st>>>(a);
-        const uint32_t gfix = grid_for(k_knn_group<32, true, false, true>, threads, smem, nchunks, t.warps_per_block);
+        const uint32_t gfix = grid_for(k_knn_group<32, true, false, true>, threads, smem, nq, t.warps_per_block, fx.rounds_per_chunk);
         k_knn_group<32, true, false, true><<<gfix, threads, smem, st>>>(fx);
         return 2;
     }
@@ -1570,19 +1653,21 @@ int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const 
     a.cap = group_capacity(p.k);
     a.smem_per_warp = (uint32_t)group_smem_bytes_per_warp(p.k, qpw);
     const int smem = (int)a.smem_per_warp * t.warps_per_block;
-    const uint32_t nchunks = (nq + (uint32_t)qpw * a.rounds_per_chunk - 1) / ((uint32_t)qpw * a.rounds_per_chunk);
+    const uint32_t rounds = (nq + (uint32_t)qpw - 1) / (uint32_t)qpw;
     a.fix_list = fix_list;
+    a.fix_bound = fix_bound;
     a.fix_count = work_counter + 1;
     a.nq_dev = nullptr;
     KnnArgs fx = a;   // fix pass: the listed queries, FP64 distances where needed
     fx.fix_in = fix_list;
     fx.nq_dev = work_counter + 1;
     fx.work_counter = work_counter + 2;
+    fx.rounds_per_chunk = 1;
 #define PM_LAUNCH_GROUP(G)                                                                          \
     {                                                                                               \
-        const uint32_t grid = grid_for(k_knn_group<G, false, false, false>, threads, smem, nchunks, t.warps_per_block); \
+        const uint32_t grid = grid_for(k_knn_group<G, false, false, false>, threads, smem, rounds, t.warps_per_block, a.rounds_per_chunk); \
         k_knn_group<G, false, false, false><<<grid, threads, smem, st>>>(a);                                      \
-        const uint32_t gfix = grid_for(k_knn_group<G, true, false, false>, threads, smem, nchunks, t.warps_per_block); \
+        const uint32_t gfix = grid_for(k_knn_group<G, true, false, false>, threads, smem, rounds, t.warps_per_block, fx.rounds_per_chunk); \
         k_knn_group<G, true, false, false><<<gfix, threads, smem, st>>>(fx);                                      \
     }
     switch (qpw) {
@@ -1599,9 +1684,9 @@ int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const 
 // the sorted query keys carry each query's map id, whose root slot and
 // parameters the kernel reads; kmax sizes the candidate buffers.
 template <bool kW>
-static int launch_batch(const MapView& m, const BatchQuery* bq, const BatchGeom* bg, uint32_t kmax, const float4* qpos,
+static int launch_batch(const MapView& m, const BatchQuery* bq, const BatchGeom* bg, uint32_t kmax, uint64_t pairs, const float4* qpos,
                     const float4* qnrm, const uint32_t* order, const uint64_t* qkeys, uint32_t nq,
-                    const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list, const QueryTuning& t,
+                    const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list, float* fix_bound, const QueryTuning& t,
                     cudaStream_t st) {
     if (!nq) return 0;
     QueryParams p;
@@ -1615,29 +1700,30 @@ static int launch_batch(const MapView& m, const BatchQuery* bq, const BatchGeom*
     a.cap = group_capacity(kmax);
     a.smem_per_warp = (uint32_t)(kW ? wide_smem_bytes_per_warp(kmax) : group_smem_bytes_per_warp(kmax, 1));
     a.fix_list = fix_list;
+    a.fix_bound = fix_bound;
     a.fix_count = work_counter + 1;
     const int threads = 32 * t.warps_per_block;
     const int smem = (int)a.smem_per_warp * t.warps_per_block;
     cudaMemsetAsync(work_counter, 0, 3 * sizeof(uint32_t), st);
-    const uint32_t nchunks = (nq + a.rounds_per_chunk - 1) / a.rounds_per_chunk;
-    const uint32_t grid = grid_for(k_knn_group<32, false, true, kW>, threads, smem, nchunks, t.warps_per_block);
-    k_knn_group<32, false, true, kW><<<grid, threads, smem, st>>>(a);
     KnnArgs fx = a;   // queries whose estimate needs FP64 distances
     fx.fix_in = fix_list;
     fx.nq_dev = work_counter + 1;
     fx.work_counter = work_counter + 2;
-    const uint32_t gfix = grid_for(k_knn_group<32, true, true, kW>, threads, smem, nchunks, t.warps_per_block);
+    fx.rounds_per_chunk = 1;
+    const uint32_t grid = grid_for(k_knn_group<32, false, true, kW>, threads, smem, nq, t.warps_per_block, a.rounds_per_chunk);
+    k_knn_group<32, false, true, kW><<<grid, threads, smem, st>>>(a);
+    const uint32_t gfix = grid_for(k_knn_group<32, true, true, kW>, threads, smem, nq, t.warps_per_block, fx.rounds_per_chunk);
     k_knn_group<32, true, true, kW><<<gfix, threads, smem, st>>>(fx);
     return 2;
 }
 
-int query_knn_batch(const MapView& m, const BatchQuery* bq, const BatchGeom* bg, uint32_t kmax, const float4* qpos,
+int query_knn_batch(const MapView& m, const BatchQuery* bq, const BatchGeom* bg, uint32_t kmax, uint64_t pairs, const float4* qpos,
                     const float4* qnrm, const uint32_t* order, const uint64_t* qkeys, uint32_t nq,
-                    const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list, const QueryTuning& t,
+                    const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list, float* fix_bound, const QueryTuning& t,
                     cudaStream_t st) {
     if (t.layout == 2)
-        return launch_batch<true>(m, bq, bg, kmax, qpos, qnrm, order, qkeys, nq, out, work_counter, fix_list, t, st);
-    return launch_batch<false>(m, bq, bg, kmax, qpos, qnrm, order, qkeys, nq, out, work_counter, fix_list, t, st);
+        return launch_batch<true>(m, bq, bg, kmax, pairs, qpos, qnrm, order, qkeys, nq, out, work_counter, fix_list, fix_bound, t, st);
+    return launch_batch<false>(m, bq, bg, kmax, pairs, qpos, qnrm, order, qkeys, nq, out, work_counter, fix_list, fix_bound, t, st);
 }
 
 int query_bruteforce(const MapView& m, const QueryParams& p, const float4* qpos, const float4* qnrm,
