@@ -415,6 +415,8 @@ def run_ours(args, cfg, light: bool = False) -> dict | None:
     kern_ms = float(np.mean(kernels))
     nodes = info.num_nodes
     alg_bytes = 48 * Q + 32 * N + 64 * (nodes + 1)
+    # sorted queries this dense share walks (pm_query.cu, shared_walk)
+    kernel = "k_knn_group" if args.unsorted or Q * k < 24 * N else "k_knn_shared"
     peak, peak_kind = measured_peaks()
     achieved = alg_bytes / (kern_ms / 1000.0) / 1e9
     build_ms = float(np.mean(builds))
@@ -435,8 +437,8 @@ def run_ours(args, cfg, light: bool = False) -> dict | None:
         "build_ms": build_ms, "build_ms_median_of_20_warm": build_median_ms, "query_ms": float(np.mean(queries)), "query_sort_ms": float(np.mean(sorts)),
         "query_kernel_ms": kern_ms, "query_only_mqueries_per_s": Q / (float(np.mean(queries)) / 1000.0) / 1e6,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": profiled_traffic("k_knn_group", args.config), "kernel": "k_knn_group",
-                     "l2_traffic": profiled_traffic("k_knn_group", args.config, "l2_bytes_per_launch"),
+                     "traffic": profiled_traffic(kernel, args.config), "kernel": kernel,
+                     "l2_traffic": profiled_traffic(kernel, args.config, "l2_bytes_per_launch"),
                      "algorithmic_bytes_per_launch": alg_bytes, "peak_source": peak_kind},
         "roofline_build": {"bound": "hbm", "achieved": build_bytes / (build_ms / 1000.0) / 1e9, "peak": peak,
                            "unit": "GB/s", "frac": build_bytes / (build_ms / 1000.0) / 1e9 / peak,

@@ -54,12 +54,14 @@ struct KnnArgs {
     float* out_r2;
     uint32_t* out_count;
     uint32_t* work_counter;
-    uint32_t* fix_list;       // sorted slots of the queries left to the fix pass (FP64 distances)
+    uint32_t* fix_list;       // sorted slots of the queries left to the fix pass (FP64 distances; the shared walk's leftovers)
     float* fix_bound;         // a bound of each listed query's search (exclusive, on d^2)
     const uint32_t* fix_in;   // fix pass: the list it works through
     uint32_t* fix_count;
     const uint32_t* nq_dev;   // fix pass: query count read on the device
     uint32_t rounds_per_chunk;   // smallest chunk of the guided schedule, in rounds
+    uint32_t rounds_max;         // longest chunk (the shared walk)
+    uint64_t neg_zero2;          // -0 twice (mul2)
     uint32_t cap;             // group kernel: candidate buffer entries per query
     uint32_t smem_per_warp;   // group kernel: shared bytes per warp
     unsigned long long* stats;   // optional traversal counters (kStat*), nullptr = off
@@ -1372,6 +1374,7 @@ __global__ void __launch_bounds__(256, kWide ? 4 : 0) k_knn_group(KnnArgs a0) {
     }
 }
 
+#include "pm_knn_shared.cuh"
 
 // Brute force: thread per query, every photon staged through shared memory.
 constexpr int kBruteThreads = 64;
@@ -1564,6 +1567,7 @@ static KnnArgs make_args(const MapView& m, const QueryParams& p, const float4* q
     a.k = p.k; a.r2max = p.r2; a.rmax = p.r; a.filter = p.filter; a.cone_k = p.cone_k; a.min_found = p.min_found;
     a.out_rad = out.rad; a.out_nbr = out.nbr; a.out_r2 = out.r2; a.out_count = out.count;
     a.work_counter = nullptr; a.rounds_per_chunk = 1;
+    a.rounds_max = 0; a.neg_zero2 = 0x8000000080000000ull;
     a.fix_list = nullptr; a.fix_bound = nullptr; a.fix_count = nullptr; a.nq_dev = nullptr; a.fix_in = nullptr;
     a.scale_ptr = &m.hdr->fix_scale;
     a.root = &m.nodes[0].c[0];
@@ -1611,6 +1615,45 @@ static uint32_t grid_for(K kernel, int threads, int smem, uint32_t rounds, int w
     return full > need ? need : full;
 }
 
+// Whether the queries are dense enough to share walks (k_knn_shared), by the
+// neighbour slots a photon.  Where they are sparse, eight queries reach too
+// many photons to stage: at 12.5 slots (65,536 photons, 16,384 queries, k = 50)
+// 0.28 ms against 0.10 one by one.  Where they are dense, sharing wins: at 198
+// (1M photons, 2M queries, k = 100) 3.12 against 5.85 ms, at 160 (400,009
+// queries, the adjoint without lists) 3.15 against 4.26 for the whole step, at
+// 64 (1M x 1M with lists and adjoint) 5.44 against 6.62, at 51 (307,200
+// queries) 1.16 against 1.18.
+static bool shared_walk(uint32_t n, uint32_t nq, uint64_t pairs) {
+    return pairs >= 24ull * n;
+}
+
+// k_knn_shared for the launch's queries (a: the wide search's arguments).
+template <bool kBatch>
+static void launch_shared(KnnArgs a, uint32_t kmax, uint32_t nq, cudaStream_t st) {
+    a.cap = shared_row(kmax);
+    a.smem_per_warp = (uint32_t)shared_smem_bytes_per_warp(kmax);
+    a.rounds_per_chunk = (a.rounds_per_chunk + 3u) / 4u;   // a round is a group of eight queries here
+    const uint32_t rounds = (nq + kShQ - 1) / kShQ;
+    // shared memory bounds the resident warps: the block size that fits most
+    auto launch = [&](auto kernel) {
+        int best = 1;
+        uint32_t most = 0;
+        for (int w = 8; w >= 4; --w) {
+            const uint32_t warps = grid_full(kernel, 32 * w, (int)a.smem_per_warp * w) * (uint32_t)w;
+            if (warps > most) { most = warps; best = w; }
+        }
+        const int smem = (int)a.smem_per_warp * best;
+        // two chunks or more per warp, of 4 to 32 groups: long chunks save searches
+        // without a bound, short ones keep a chunk in a dense blob from outlasting
+        // the rest
+        a.rounds_max = std::min(32u, std::max(4u, rounds / (2u * std::max(1u, most))));
+        const uint32_t grid = grid_for(kernel, 32 * best, smem, rounds, best, a.rounds_per_chunk);
+        kernel<<<grid, 32 * best, smem, st>>>(a);
+    };
+    if (a.out_nbr) launch(k_knn_shared<kBatch, true>);
+    else launch(k_knn_shared<kBatch, false>);
+}
+
 int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const float4* qnrm,
               const uint32_t* order, uint32_t nq, const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list, float* fix_bound,
               const QueryTuning& t, cudaStream_t st) {
@@ -1643,8 +1686,12 @@ int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const 
         fx.work_counter = work_counter + 2;
         fx.rounds_per_chunk = 1;
         fx.qsorted = nullptr;
-        const uint32_t grid = grid_for(k_knn_group<32, false, false, true>, threads, smem, nq, t.warps_per_block, a.rounds_per_chunk);
-        k_knn_group<32, false, false, true><<<grid, threads, smem, st>>>(a);
+        if (order && shared_walk(m.n, nq, (uint64_t)nq * p.k)) {
+            launch_shared<false>(a, p.k, nq, st);
+        } else {
+            const uint32_t grid = grid_for(k_knn_group<32, false, false, true>, threads, smem, nq, t.warps_per_block, a.rounds_per_chunk);
+            k_knn_group<32, false, false, true><<<grid, threads, smem, st>>>(a);
+        }
         const uint32_t gfix = grid_for(k_knn_group<32, true, false, true>, threads, smem, nq, t.warps_per_block, fx.rounds_per_chunk);
         k_knn_group<32, true, false, true><<<gfix, threads, smem, st>>>(fx);
         return 2;
@@ -1705,13 +1752,18 @@ static int launch_batch(const MapView& m, const BatchQuery* bq, const BatchGeom*
     const int threads = 32 * t.warps_per_block;
     const int smem = (int)a.smem_per_warp * t.warps_per_block;
     cudaMemsetAsync(work_counter, 0, 3 * sizeof(uint32_t), st);
-    KnnArgs fx = a;   // queries whose estimate needs FP64 distances
+    KnnArgs fx = a;   // queries whose estimate needs FP64 distances, or that the shared walk left
     fx.fix_in = fix_list;
     fx.nq_dev = work_counter + 1;
     fx.work_counter = work_counter + 2;
     fx.rounds_per_chunk = 1;
-    const uint32_t grid = grid_for(k_knn_group<32, false, true, kW>, threads, smem, nq, t.warps_per_block, a.rounds_per_chunk);
-    k_knn_group<32, false, true, kW><<<grid, threads, smem, st>>>(a);
+    if (kW && shared_walk(m.n, nq, pairs)) {
+        a.qsorted = t.qsorted;
+        launch_shared<true>(a, kmax, nq, st);
+    } else {
+        const uint32_t grid = grid_for(k_knn_group<32, false, true, kW>, threads, smem, nq, t.warps_per_block, a.rounds_per_chunk);
+        k_knn_group<32, false, true, kW><<<grid, threads, smem, st>>>(a);
+    }
     const uint32_t gfix = grid_for(k_knn_group<32, true, true, kW>, threads, smem, nq, t.warps_per_block, fx.rounds_per_chunk);
     k_knn_group<32, true, true, kW><<<gfix, threads, smem, st>>>(fx);
     return 2;
