@@ -514,17 +514,6 @@ pm_status pm_query(pm_map* m, const pm_query_desc* desc, const float* d_qpos4, c
     return query_exact_run(m, desc, d_qpos4, d_qnrm4, nq, d_rad4, d_nbr, d_r2, d_count, st, nullptr);
 }
 
-// Device address of a page-locked host array (cudaHostAlloc /
-// cudaHostRegister, mapped under unified addressing), or nullptr.
-static void* host_mapped(const void* p) {
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
-}
-
 pm_status pm_build_query_host(pm_map* m, const float* h_pos4, const float* h_pow4, uint32_t n, int format,
                               const pm_query_desc* desc, const float* h_qpos4, const float* h_qnrm4, uint32_t nq,
                               float* h_rad4, uint32_t chunks, void* stream) {
@@ -561,16 +550,6 @@ pm_status pm_build_query_host(pm_map* m, const float* h_pos4, const float* h_pow
     float4* dqp = P<float4>(m->hs_qpos);
     float4* dqn = P<float4>(m->hs_qnrm);
     float4* drad = P<float4>(m->hs_rad);
-    // A page-locked, 16-byte aligned radiance array is written in place by the query kernel
-    // (each estimate once, 16 bytes over PCIe while the search runs), which
-    // takes the download off the critical path: 9.83 -> 9.27 ms end to end on
-    // the plain workload.  A pageable one goes through a device copy.  The
-    // normals are always copied in: read in place as well, they queue behind
-    // the posted radiance writes on the link (12.76 ms with both in place;
-    // 9.57 ms with the normals alone).
-    void* const rad_mapped = (nq > 0 && aligned16(h_rad4)) ? host_mapped(h_rad4) : nullptr;
-    const bool rad_in_place = rad_mapped != nullptr;
-    if (rad_in_place) drad = reinterpret_cast<float4*>(rad_mapped);
     cudaEvent_t ev_photons = m->hs_ev[0], ev_done = m->hs_ev[1];
     // photons in, then the queries in pieces behind them on the copy stream
     if (n) {
@@ -599,7 +578,10 @@ pm_status pm_build_query_host(pm_map* m, const float* h_pos4, const float* h_pow
     if (s != PM_OK) return s;
     if (!m->built) return fail(m, PM_ERR_STATE, "no photon map has been built");
     // each piece is sorted once its positions have arrived and searched once
-    // its normals have; its radiance leaves on the second stream
+    // its normals have; its radiance leaves on the second stream.  (The search
+    // writing a pinned h_rad4 in place, 16 bytes a query over PCIe, is bound by
+    // those writes: 7.93 ms end to end against 7.41 with the copy, 1M photons and
+    // 2M queries.)
     for (uint32_t c = 0; c < chunks; ++c) {
         const size_t off = bounds[c], len = bounds[c + 1] - bounds[c];
         cudaStreamWaitEvent(st, m->hs_ev[2 + 3 * c], 0);
@@ -613,7 +595,7 @@ pm_status pm_build_query_host(pm_map* m, const float* h_pos4, const float* h_pow
         }
         cudaEventRecord(m->hs_ev[4 + 3 * c], st);
         cudaStreamWaitEvent(m->hs_out, m->hs_ev[4 + 3 * c], 0);
-        if (len && !rad_in_place)
+        if (len)
             cudaMemcpyAsync(reinterpret_cast<float4*>(h_rad4) + off, drad + off, len * sizeof(float4),
                             cudaMemcpyDeviceToHost, m->hs_out);
     }
