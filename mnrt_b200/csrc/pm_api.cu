@@ -1349,7 +1349,7 @@ pm_status batch_build_device(pm_batch* b, const float* d_pos4, const float* d_po
     return check_cuda(m, "pm_batch_build");
 }
 
-pm_status batch_query_device(pm_batch* b, uint32_t kmax, uint64_t pairs, const float* d_qpos4, const float* d_qnrm4, uint32_t nq,
+pm_status batch_query_device(pm_batch* b, uint32_t kmax, const float* d_qpos4, const float* d_qnrm4, uint32_t nq,
                              float* d_rad4, uint32_t* d_nbr, float* d_r2, uint32_t* d_count, cudaStream_t st) {
     pm_map* m = b->m;
     if (nq == 0) return PM_OK;
@@ -1370,7 +1370,7 @@ pm_status batch_query_device(pm_batch* b, uint32_t kmax, uint64_t pairs, const f
     }
     MapView v = view_of(m);
     v.n = b->total_photons;
-    nl += query_knn_batch(v, P<BatchQuery>(b->bq), P<BatchGeom>(b->geom), kmax, pairs, qpos,
+    nl += query_knn_batch(v, P<BatchQuery>(b->bq), P<BatchGeom>(b->geom), kmax, qpos,
                           reinterpret_cast<const float4*>(d_qnrm4), vals[cur], keys[cur], nq, out, P<uint32_t>(m->counter),
                           P<uint32_t>(m->fixq), reinterpret_cast<float*>(keys[cur ^ 1]), t, st);
     m->launches += (uint64_t)nl;
@@ -1469,7 +1469,7 @@ pm_status pm_batch_query(pm_batch* b, const pm_query_desc* descs, const float* d
     if (s != PM_OK) return s;
     if ((s = ensure_query_capacity(b->m, nq, st)) != PM_OK) return s;
     if ((s = batch_upload_queries(b, descs, query_offsets, &kmax, &nbr_total)) != PM_OK) return s;
-    return batch_query_device(b, kmax, nbr_total, d_qpos4, d_qnrm4, nq, d_rad4, d_nbr, d_r2, d_count, st);
+    return batch_query_device(b, kmax, d_qpos4, d_qnrm4, nq, d_rad4, d_nbr, d_r2, d_count, st);
 }
 
 pm_status pm_batch_capture(pm_batch* b, const float* d_pos4, const float* d_pow4, const uint32_t* photon_offsets,
@@ -1493,7 +1493,7 @@ pm_status pm_batch_capture(pm_batch* b, const float* d_pos4, const float* d_pow4
     if (cudaStreamBeginCapture(b->cap_stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
         return check_cuda(b->m, "pm_batch_capture: begin");
     pm_status sb = batch_build_device(b, d_pos4, d_pow4, format, b->cap_stream);
-    pm_status sq = sb == PM_OK ? batch_query_device(b, kmax, nbr_total, d_qpos4, d_qnrm4, nq, d_rad4, d_nbr, d_r2, d_count,
+    pm_status sq = sb == PM_OK ? batch_query_device(b, kmax, d_qpos4, d_qnrm4, nq, d_rad4, d_nbr, d_r2, d_count,
                                                     b->cap_stream)
                                : sb;
     cudaGraph_t g = nullptr;

@@ -190,7 +190,7 @@ int query_bruteforce(const MapView& m, const QueryParams& p, const float4* qpos,
 int query_smem_bytes_per_warp(uint32_t k);
 double filter_norm_const(int filter, float cone_k);
 
-int query_knn_batch(const MapView& m, const BatchQuery* bq, const BatchGeom* bg, uint32_t kmax, uint64_t pairs, const float4* qpos,
+int query_knn_batch(const MapView& m, const BatchQuery* bq, const BatchGeom* bg, uint32_t kmax, const float4* qpos,
                     const float4* qnrm, const uint32_t* order, const uint64_t* qkeys, uint32_t nq,
                     const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list, float* fix_bound, const QueryTuning& t,
                     cudaStream_t st);

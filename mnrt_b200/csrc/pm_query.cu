@@ -1615,16 +1615,19 @@ static uint32_t grid_for(K kernel, int threads, int smem, uint32_t rounds, int w
     return full > need ? need : full;
 }
 
-// Whether the queries are dense enough to share walks (k_knn_shared), by the
-// neighbour slots a photon.  Where they are sparse, eight queries reach too
-// many photons to stage: at 12.5 slots (65,536 photons, 16,384 queries, k = 50)
-// 0.28 ms against 0.10 one by one.  Where they are dense, sharing wins: at 198
-// (1M photons, 2M queries, k = 100) 3.12 against 5.85 ms, at 160 (400,009
-// queries, the adjoint without lists) 3.15 against 4.26 for the whole step, at
-// 64 (1M x 1M with lists and adjoint) 5.44 against 6.62, at 51 (307,200
-// queries) 1.16 against 1.18.
-static bool shared_walk(uint32_t n, uint32_t nq, uint64_t pairs) {
-    return pairs >= 24ull * n;
+// Whether enough queries are at hand to share walks (k_knn_shared).  Eight
+// queries cost less together, but a launch's longest warp takes longer (a chunk
+// in a dense blob: 0.3 ms with 65,536 photons, 0.9 with 1M), and sparse queries
+// reach more photons than fit.  One by one / shared, ms (R = 0.1, cone):
+//   65,536 photons:  k = 16: 131,072 queries 0.31 / 0.34, 262,144 0.52 / 0.42;
+//                    k = 100: 62,914 0.29 / 0.40
+//   300,001 photons: k = 16: 300,001 0.64 / 0.70, 450,001 0.90 / 0.75;
+//                    k = 100: 144,000 0.56 / 0.84, 288,000 0.95 / 0.95
+//   1M photons:      k = 50: 503,316 1.29 / 1.26, 1,006,632 2.36 / 1.57;
+//                    k = 100: 503,316 1.65 / 1.87, 671,088 2.11 / 2.08, 1,006,632 3.02 / 2.22
+// The line follows the break-even points: 640 sqrt(photons), 262,144 at least.
+static bool shared_walk(uint32_t n, uint32_t nq) {
+    return nq >= 262144u && (uint64_t)nq * nq >= 409600ull * n;
 }
 
 // k_knn_shared for the launch's queries (a: the wide search's arguments).
@@ -1686,7 +1689,7 @@ int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const 
         fx.work_counter = work_counter + 2;
         fx.rounds_per_chunk = 1;
         fx.qsorted = nullptr;
-        if (order && shared_walk(m.n, nq, (uint64_t)nq * p.k)) {
+        if (order && shared_walk(m.n, nq)) {
             launch_shared<false>(a, p.k, nq, st);
         } else {
             const uint32_t grid = grid_for(k_knn_group<32, false, false, true>, threads, smem, nq, t.warps_per_block, a.rounds_per_chunk);
@@ -1731,7 +1734,7 @@ int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const 
 // the sorted query keys carry each query's map id, whose root slot and
 // parameters the kernel reads; kmax sizes the candidate buffers.
 template <bool kW>
-static int launch_batch(const MapView& m, const BatchQuery* bq, const BatchGeom* bg, uint32_t kmax, uint64_t pairs, const float4* qpos,
+static int launch_batch(const MapView& m, const BatchQuery* bq, const BatchGeom* bg, uint32_t kmax, const float4* qpos,
                     const float4* qnrm, const uint32_t* order, const uint64_t* qkeys, uint32_t nq,
                     const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list, float* fix_bound, const QueryTuning& t,
                     cudaStream_t st) {
@@ -1757,7 +1760,7 @@ static int launch_batch(const MapView& m, const BatchQuery* bq, const BatchGeom*
     fx.nq_dev = work_counter + 1;
     fx.work_counter = work_counter + 2;
     fx.rounds_per_chunk = 1;
-    if (kW && shared_walk(m.n, nq, pairs)) {
+    if (kW && shared_walk(m.n, nq)) {
         a.qsorted = t.qsorted;
         launch_shared<true>(a, kmax, nq, st);
     } else {
@@ -1769,13 +1772,13 @@ static int launch_batch(const MapView& m, const BatchQuery* bq, const BatchGeom*
     return 2;
 }
 
-int query_knn_batch(const MapView& m, const BatchQuery* bq, const BatchGeom* bg, uint32_t kmax, uint64_t pairs, const float4* qpos,
+int query_knn_batch(const MapView& m, const BatchQuery* bq, const BatchGeom* bg, uint32_t kmax, const float4* qpos,
                     const float4* qnrm, const uint32_t* order, const uint64_t* qkeys, uint32_t nq,
                     const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list, float* fix_bound, const QueryTuning& t,
                     cudaStream_t st) {
     if (t.layout == 2)
-        return launch_batch<true>(m, bq, bg, kmax, pairs, qpos, qnrm, order, qkeys, nq, out, work_counter, fix_list, fix_bound, t, st);
-    return launch_batch<false>(m, bq, bg, kmax, pairs, qpos, qnrm, order, qkeys, nq, out, work_counter, fix_list, fix_bound, t, st);
+        return launch_batch<true>(m, bq, bg, kmax, qpos, qnrm, order, qkeys, nq, out, work_counter, fix_list, fix_bound, t, st);
+    return launch_batch<false>(m, bq, bg, kmax, qpos, qnrm, order, qkeys, nq, out, work_counter, fix_list, fix_bound, t, st);
 }
 
 int query_bruteforce(const MapView& m, const QueryParams& p, const float4* qpos, const float4* qnrm,

@@ -1,4 +1,4 @@
-"""Sorted queries that are dense against the photons share walks of the tree
+"""Sorted queries of large sets share walks of the tree
 (k_knn_shared); queries in the given order are searched one by one.  Every
 output of the two must have the same bits: the neighbour sets are exact and the
 flux sums do not depend on the order of their terms."""
@@ -30,19 +30,19 @@ def both(pm, qp, qn, nbr=True, **kw):
 
 
 CASES = [
-    # n, nq, k, R, filter, caustic, cluster, leaf (nq k >= 24 n: walks are shared)
-    (1, 24, 1, 0.5, "box", 0.0, 0.0, 32),
-    (2, 49, 2, 2.0, "cone", 0.0, 0.0, 1),
-    (40, 1000, 128, 3.0, "epanechnikov", 0.0, 0.0, 64),       # fewer photons than k
-    (64, 1537, 1, 0.2, "cone", 0.0, 0.0, 64),
-    (65, 1561, 31, 0.5, "cone", 0.0, 0.0, 64),
-    (3000, 2257, 32, 0.1, "cone", 0.0, 0.0, 32),
-    (3000, 2263, 33, 0.1, "epanechnikov", 0.2, 0.0, 7),
-    (20000, 8001, 64, 0.05, "epanechnikov", 0.2, 0.5, 64),
-    (20000, 8007, 65, 0.05, "cone", 0.2, 0.5, 32),
-    (50000, 30001, 100, 0.1, "cone", 0.2, 0.0, 64),
-    (50000, 30000, 128, 0.02, "box", 0.9, 0.5, 33),           # dense blob: queries left to the fix pass
-    (30000, 100003, 8, 0.01, "cone", 0.2, 0.5, 64),           # R the bound of most queries
+    # n, nq, k, R, filter, caustic, cluster, leaf (262,144 queries and more: walks are shared)
+    (1, 262144, 1, 0.5, "box", 0.0, 0.0, 32),
+    (2, 262145, 2, 2.0, "cone", 0.0, 0.0, 1),
+    (40, 262151, 128, 3.0, "epanechnikov", 0.0, 0.0, 64),     # fewer photons than k
+    (64, 262147, 1, 0.2, "cone", 0.0, 0.0, 64),
+    (65, 262145, 31, 0.5, "cone", 0.0, 0.0, 64),
+    (3000, 262150, 32, 0.1, "cone", 0.0, 0.0, 32),
+    (3000, 262149, 33, 0.1, "epanechnikov", 0.2, 0.0, 7),
+    (20000, 262145, 64, 0.05, "epanechnikov", 0.2, 0.5, 64),
+    (100000, 262151, 65, 0.05, "cone", 0.2, 0.5, 32),
+    (150000, 262145, 100, 0.1, "cone", 0.2, 0.0, 64),
+    (50000, 262144, 128, 0.02, "box", 0.9, 0.5, 33),          # dense blob: queries left to the fix pass
+    (30000, 262147, 8, 0.01, "cone", 0.2, 0.5, 64),           # R the bound of most queries
 ]
 
 
@@ -62,7 +62,7 @@ def test_shared_walk_is_the_single_search(cuda, n, nq, k, r, filt, caustic, clus
 @pytest.mark.parametrize("copies", [2, 40, 1000])
 def test_shared_walk_ties(cuda, copies):
     """Photons in `copies` places at once: the k-th distance is a tie of many."""
-    n, nq, k = 4000, 3000, 50
+    n, nq, k = 4000, 262147, 50
     ph = gen.photons(n, seed=3, caustic_frac=0.0)
     ph.pos[:, :3] = np.tile(ph.pos[: n // copies, :3], (copies, 1))
     q = gen.queries(nq, seed=4)
@@ -79,7 +79,7 @@ def test_shared_walk_clumps(cuda, clump, nbr):
     that do not fit, halve, and grow back must still answer every query once."""
     n, k = 60000, 128
     ph = gen.photons(n, seed=8, caustic_frac=0.2)
-    at = gen.queries(4000, seed=9).pos[:, :3]
+    at = gen.queries(262144 // clump + 1, seed=9).pos[:, :3]
     rng = np.random.default_rng(clump)
     pos = np.zeros((len(at) * clump, 4), np.float32)
     pos[:, :3] = np.repeat(at, clump, 0) + rng.uniform(-0.02, 0.02, (len(at) * clump, 3)).astype(np.float32)
@@ -91,7 +91,7 @@ def test_shared_walk_clumps(cuda, clump, nbr):
 
 
 def test_shared_walk_in_a_batch(cuda):
-    sizes = [(0, 50), (3, 700), (500, 1), (9000, 9001), (1, 60), (20000, 12345), (64, 0)]
+    sizes = [(0, 50), (3, 700), (500, 1), (9000, 120001), (1, 60), (20000, 171345), (64, 0)]
     ks = [16, 128, 5, 64, 32, 100, 7]
     ph = [gen.photons(n, seed=10 + i, caustic_frac=0.2 if n > 100 else 0.0) for i, (n, _) in enumerate(sizes)]
     q = [gen.queries(m, seed=30 + i) for i, (_, m) in enumerate(sizes)]
