@@ -1590,9 +1590,22 @@ int group_smem_bytes_per_warp(uint32_t k, int qpw) {
            kStackDepth * (int)sizeof(uint32_t);
 }
 
+// A kernel's limit on dynamic shared memory belongs to the process, and handles
+// are queried from several threads: it is raised to the device's maximum (these
+// kernels have no static shared memory) and never follows a launch's size, which
+// would lower it between another thread's set and launch.
+template <class K>
+static void allow_smem(K kernel, int smem) {
+    if (smem <= 48 * 1024) return;
+    int dev = 0, most = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 template <class K>
 static uint32_t grid_full(K kernel, int threads, int smem) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    allow_smem(kernel, smem);
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1786,7 +1799,7 @@ int query_bruteforce(const MapView& m, const QueryParams& p, const float4* qpos,
     if (!nq) return 0;
     KnnArgs a = make_args(m, p, qpos, qnrm, nullptr, nq, out);
     const int smem = kBruteTile * (int)sizeof(float4) + kBruteThreads * (int)p.k * (int)sizeof(uint64_t);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_knn_brute, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    allow_smem(k_knn_brute, smem);
     k_knn_brute<<<(nq + kBruteThreads - 1) / kBruteThreads, kBruteThreads, smem, st>>>(a, m.n);
     return 1;
 }

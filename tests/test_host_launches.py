@@ -1,0 +1,104 @@
+"""The engine's host code without a GPU: its sources linked with a CUDA runtime
+that keeps a log instead of launching (tests/cpp/host_runtime.cpp).  Shows what
+a call asks the runtime for, and what it does when the runtime refuses."""
+import ctypes as C
+import shutil
+import subprocess
+import threading
+from concurrent.futures import ThreadPoolExecutor
+from pathlib import Path
+
+import pytest
+
+from mnrt_b200 import _lib as L
+from mnrt_b200 import build
+
+HERE = Path(__file__).resolve().parent
+
+
+class Engine:
+    """The host-only library: handles, calls and the runtime's log."""
+
+    def __init__(self, path):
+        self.lib = L.load(path)
+        self.lib.host_log.restype = C.c_char_p
+        self.lib.host_set.argtypes = [C.c_char_p, C.c_int]
+
+    def log(self):
+        return self.lib.host_log().decode().splitlines()
+
+    def set(self, name, value):
+        self.lib.host_set(name.encode(), value)
+
+    def map(self, n, nq=0):
+        h = C.c_void_p()
+        assert self.lib.pm_create(C.byref(h), 0, None, None, 0.1) == L.PM_OK
+        assert self.lib.pm_reserve(h, n, nq) == L.PM_OK
+        return h
+
+    def build(self, h, n):   # the photon arrays are never read: nothing is launched
+        return self.lib.pm_build(h, 16, 32, n, L.PM_PHOTONS_PACKED, None)
+
+    def query(self, h, nq, call="pm_query", **kw):
+        return getattr(self.lib, call)(h, C.byref(desc(**kw)), 16, 32, nq, 48, None, None, None, None)
+
+
+def desc(**kw):
+    return L.QueryDesc(**{**dict(k=50, r_max=0.1, filter=L.PM_FILTER_CONE, cone_k=1.0, mode=L.PM_MODE_EXACT, min_found=0,
+                                 order=L.PM_ORDER_SORTED, refine_iters=2), **kw})
+
+
+def launched(log, name):
+    return [x for x in log if x.split()[0] in ("launch", "cluster") and x.split()[1].startswith(name)]
+
+
+@pytest.fixture(scope="module")
+def engine(tmp_path_factory):
+    tmp = tmp_path_factory.mktemp("host")
+
+    def compile(src):   # PTX only: nothing of it runs
+        out = tmp / (src + ".o")
+        cmd = [build.nvcc(), "-gencode", "arch=compute_100a,code=compute_100a", "-Xcicc", "-O0", "-w", "-std=c++17",
+               "--expt-relaxed-constexpr", "-cudart", "none", "-Xcompiler", "-fPIC,-fvisibility=hidden", "-I",
+               str(build.ROOT / "include"), "-c", str(build.CSRC / src), "-o", str(out)]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        assert r.returncode == 0, r.stderr
+        return str(out)
+
+    with ThreadPoolExecutor(8) as pool:
+        objects = list(pool.map(compile, build.SOURCES))
+    lib = tmp / "libpmgpu_host.so"
+    cuda = Path(shutil.which("nvcc") or build.nvcc()).resolve().parent.parent
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-fvisibility=hidden", "-I", str(cuda / "include"),
+                        str(HERE / "cpp" / "host_runtime.cpp"), *objects, "-Wl,--no-undefined", "-o", str(lib)],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    return Engine(lib)
+
+
+@pytest.mark.parametrize("call,kernel", [("pm_query", "k_knn_shared"), ("pm_query_bruteforce", "k_knn_brute")])
+def test_shared_memory_limit_is_never_lowered(engine, call, kernel):
+    """A kernel's limit on dynamic shared memory belongs to the process: a call
+    that lowers it, even for a moment, fails the launches of other threads."""
+    n, nq = 1000, 262144
+    handles = [engine.map(n, nq) for _ in range(2)]
+    for h in handles:
+        assert engine.build(h, n) == L.PM_OK
+    engine.log()
+    status = []
+
+    def work(h, k):
+        for _ in range(200):
+            status.append(engine.query(h, nq, call, k=k))
+
+    threads = [threading.Thread(target=work, args=(h, k)) for h, k in zip(handles, (100, 128))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    log = engine.log()
+    assert launched(log, kernel)
+    assert not [x for x in log if x.startswith(("lowered", "refused"))]
+    assert set(status) == {L.PM_OK}
+    for h in handles:
+        engine.lib.pm_destroy(h)
