@@ -50,6 +50,7 @@ struct pm_map {
     // query-sized
     DevBuf qkeys0, qkeys1, qvals0, qvals1, qscratch, counter, fixq, qsorted;
     DevBuf stats;           // query counters (profiling level 2)
+    uint32_t shared_shapes[kSharedShapes] = {};   // QueryTuning::shared_shapes
     // backward (pm_query_backward): pair sort, per-query records, segments,
     // FP64 running sums, and the forward outputs when the kNN is recomputed
     DevBuf bvals, bvals1, bkeys0, bkeys1, bscratch, blong, qrec, bphoton, seg_start, seg_end, acc;
@@ -259,8 +260,9 @@ WideBuffers wide_of(pm_map* m) {
     return w;
 }
 
-QueryTuning tuning_of(const pm_map* m) {
+QueryTuning tuning_of(pm_map* m) {
     QueryTuning t;
+    t.shared_shapes = m->shared_shapes;
     t.layout = m->kbuf_layout;
     t.queries_per_warp = m->queries_per_warp;
     t.warps_per_block = m->warps_per_block;

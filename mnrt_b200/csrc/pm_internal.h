@@ -173,12 +173,14 @@ const uint32_t* query_order(const float4* qpos, uint32_t nq, const MapHeader* hd
                             const float4* qnrm = nullptr, float4* recs = nullptr);
 constexpr int kQueryKeyBits = 30;         // bits of the query Hilbert keys (sorted as uint32)
 constexpr int kBatchQueryMapShift = 30;   // batch query keys: (map id << 30) | 30-bit Hilbert index in the map's cell
+constexpr uint32_t kSharedShapes = 2 * (kMaxK + 1);   // by k, without and with neighbour lists
 struct QueryTuning {
     int layout;             // 0: lane per query with a shared-memory heap; 1: group buffers
     int queries_per_warp;   // group layout: 1, 2, 4 or 8 (32, 16, 8 or 4 lanes per query)
     int warps_per_block;
     int rounds_per_chunk;
     unsigned long long* stats;   // 8 traversal counters (group layout), nullptr = off
+    uint32_t* shared_shapes;     // the handle's launch shapes of the shared walk (kSharedShapes words, 0: not asked yet)
     const float4* qsorted = nullptr;   // query records in sorted order (pos.xyz | caller index, normal), or nullptr
 };
 int gather_queries(const uint32_t* order, const float4* qpos, const float4* qnrm, uint32_t nq, float4* out, cudaStream_t st);

@@ -1618,14 +1618,16 @@ static uint32_t grid_full(K kernel, int threads, int smem) {
 // lowered: a launch this small is bound by its longest warp, and a query
 // without its predecessor's radius bound costs less than waiting for it (4,095
 // queries, 1M photons, k = 100: 183 -> 58 us).
-template <class K>
-static uint32_t grid_for(K kernel, int threads, int smem, uint32_t rounds, int warps_per_block, uint32_t& chunk) {
-    const uint32_t full = grid_full(kernel, threads, smem);
+static uint32_t grid_of(uint32_t full, uint32_t rounds, int warps_per_block, uint32_t& chunk) {
     const uint32_t fair = rounds / (full * (uint32_t)warps_per_block);
     if (chunk > fair) chunk = fair > 1 ? fair : 1;
     const uint32_t chunks = (rounds + chunk - 1) / chunk;
     const uint32_t need = (chunks + warps_per_block - 1) / warps_per_block;
     return full > need ? need : full;
+}
+template <class K>
+static uint32_t grid_for(K kernel, int threads, int smem, uint32_t rounds, int warps_per_block, uint32_t& chunk) {
+    return grid_of(grid_full(kernel, threads, smem), rounds, warps_per_block, chunk);
 }
 
 // Whether enough queries are at hand to share walks (k_knn_shared).  Eight
@@ -1645,26 +1647,30 @@ static bool shared_walk(uint32_t n, uint32_t nq) {
 
 // k_knn_shared for the launch's queries (a: the wide search's arguments).
 template <bool kBatch>
-static void launch_shared(KnnArgs a, uint32_t kmax, uint32_t nq, cudaStream_t st) {
+static void launch_shared(KnnArgs a, uint32_t kmax, uint32_t nq, uint32_t* shapes, cudaStream_t st) {
     a.cap = shared_row(kmax);
     a.smem_per_warp = (uint32_t)shared_smem_bytes_per_warp(kmax);
     a.rounds_per_chunk = (a.rounds_per_chunk + 3u) / 4u;   // a round is a group of eight queries here
     const uint32_t rounds = (nq + kShQ - 1) / kShQ;
-    // shared memory bounds the resident warps: the block size that fits most
+    uint32_t& shape = shapes[(a.out_nbr ? kMaxK + 1u : 0u) + kmax];
     auto launch = [&](auto kernel) {
-        int best = 1;
-        uint32_t most = 0;
-        for (int w = 8; w >= 4; --w) {
-            const uint32_t warps = grid_full(kernel, 32 * w, (int)a.smem_per_warp * w) * (uint32_t)w;
-            if (warps > most) { most = warps; best = w; }
+        // shared memory bounds the resident warps: the block size that fits most.
+        // Asked once for a handle and k (five occupancy queries).
+        if (!shape) {
+            uint32_t best = 1, most = 0;
+            for (uint32_t w = 8; w >= 4; --w) {
+                const uint32_t full = grid_full(kernel, 32 * (int)w, (int)(a.smem_per_warp * w));
+                if (full * w > most) { most = full * w; best = w; }
+            }
+            shape = most << 4 | best;
         }
-        const int smem = (int)a.smem_per_warp * best;
+        const uint32_t warps = shape & 15u, most = shape >> 4;
         // two chunks or more per warp, of 4 to 32 groups: long chunks save searches
         // without a bound, short ones keep a chunk in a dense blob from outlasting
         // the rest
-        a.rounds_max = std::min(32u, std::max(4u, rounds / (2u * std::max(1u, most))));
-        const uint32_t grid = grid_for(kernel, 32 * best, smem, rounds, best, a.rounds_per_chunk);
-        kernel<<<grid, 32 * best, smem, st>>>(a);
+        a.rounds_max = std::min(32u, std::max(4u, rounds / (2u * most)));
+        const uint32_t grid = grid_of(most / warps, rounds, (int)warps, a.rounds_per_chunk);
+        kernel<<<grid, 32 * warps, a.smem_per_warp * warps, st>>>(a);
     };
     if (a.out_nbr) launch(k_knn_shared<kBatch, true>);
     else launch(k_knn_shared<kBatch, false>);
@@ -1703,7 +1709,7 @@ int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const 
         fx.rounds_per_chunk = 1;
         fx.qsorted = nullptr;
         if (order && shared_walk(m.n, nq)) {
-            launch_shared<false>(a, p.k, nq, st);
+            launch_shared<false>(a, p.k, nq, t.shared_shapes, st);
         } else {
             const uint32_t grid = grid_for(k_knn_group<32, false, false, true>, threads, smem, nq, t.warps_per_block, a.rounds_per_chunk);
             k_knn_group<32, false, false, true><<<grid, threads, smem, st>>>(a);
@@ -1775,7 +1781,7 @@ static int launch_batch(const MapView& m, const BatchQuery* bq, const BatchGeom*
     fx.rounds_per_chunk = 1;
     if (kW && shared_walk(m.n, nq)) {
         a.qsorted = t.qsorted;
-        launch_shared<true>(a, kmax, nq, st);
+        launch_shared<true>(a, kmax, nq, t.shared_shapes, st);
     } else {
         const uint32_t grid = grid_for(k_knn_group<32, false, true, kW>, threads, smem, nq, t.warps_per_block, a.rounds_per_chunk);
         k_knn_group<32, false, true, kW><<<grid, threads, smem, st>>>(a);

@@ -39,8 +39,8 @@ class Engine:
     def build(self, h, n):   # the photon arrays are never read: nothing is launched
         return self.lib.pm_build(h, 16, 32, n, L.PM_PHOTONS_PACKED, None)
 
-    def query(self, h, nq, call="pm_query", **kw):
-        return getattr(self.lib, call)(h, C.byref(desc(**kw)), 16, 32, nq, 48, None, None, None, None)
+    def query(self, h, nq, call="pm_query", lists=False, **kw):
+        return getattr(self.lib, call)(h, C.byref(desc(**kw)), 16, 32, nq, 48, 64 if lists else None, None, None, None)
 
 
 def desc(**kw):
@@ -102,3 +102,19 @@ def test_shared_memory_limit_is_never_lowered(engine, call, kernel):
     assert set(status) == {L.PM_OK}
     for h in handles:
         engine.lib.pm_destroy(h)
+
+
+@pytest.mark.parametrize("lists", [False, True])
+def test_shared_walk_asks_for_its_block_size_once(engine, lists):
+    n, nq = 1000, 262144
+    h = engine.map(n, nq)
+    assert engine.build(h, n) == L.PM_OK
+    asked = []
+    for k in (100, 100, 128, 100, 128):
+        engine.log()
+        assert engine.query(h, nq, lists=lists, k=k) == L.PM_OK
+        log = engine.log()
+        assert len(launched(log, "k_knn_shared")) == 1
+        asked.append(sum(x.startswith("occupancy k_knn_shared") for x in log))
+    assert asked == [5, 0, 5, 0, 0]
+    engine.lib.pm_destroy(h)
