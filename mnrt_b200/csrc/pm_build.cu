@@ -603,12 +603,14 @@ int build_map(const float4* in_pos, const float4* in_pow, uint32_t n, int format
     // the last sort pass moves the photons into tree order (n >= 2; one photon is not sorted)
     const SortGather g{in_pos, in_pow, format, out_pos, out_pow, inv};
     const bool fuse = n > 1 && n <= kGatherInSortMax;
+    bool sorted = false;
     if (n > 1 && n <= kSmallSortMax) {
-        if (n <= kSmallSortMax / 4) launch_small_sort<uint64_t, 1>(k_small_build<1>, n, st, in_pos, in_pow, n, g, keys[0], hdr);
-        else if (n <= kSmallSortMax / 2) launch_small_sort<uint64_t, 2>(k_small_build<2>, n, st, in_pos, in_pow, n, g, keys[0], hdr);
-        else launch_small_sort<uint64_t, 4>(k_small_build<4>, n, st, in_pos, in_pow, n, g, keys[0], hdr);
-        ++nl;
-    } else {
+        if (n <= kSmallSortMax / 4) sorted = launch_small_sort<uint64_t, 1>(k_small_build<1>, n, st, in_pos, in_pow, n, g, keys[0], hdr);
+        else if (n <= kSmallSortMax / 2) sorted = launch_small_sort<uint64_t, 2>(k_small_build<2>, n, st, in_pos, in_pow, n, g, keys[0], hdr);
+        else sorted = launch_small_sort<uint64_t, 4>(k_small_build<4>, n, st, in_pos, in_pow, n, g, keys[0], hdr);
+        if (sorted) ++nl;
+    }
+    if (!sorted) {
         const uint32_t nb = (uint32_t)((n + kBoundsThreads - 1) / kBoundsThreads);
         const uint32_t bblocks = nb < 1 ? 1 : (nb > (uint32_t)kBoundsBlocksMax ? (uint32_t)kBoundsBlocksMax : nb);
         cudaMemsetAsync(&hdr->errors, 0, sizeof(uint32_t), st);

@@ -159,12 +159,14 @@ inline uint32_t small_sort_blocks(uint32_t n, int R) {
     return b;
 }
 
-// Launches `kernel` (which calls small_sort<Key, R>) as one cluster.
+// Launches `kernel` (which calls small_sort<Key, R>) as one cluster.  False, with
+// nothing enqueued and no error left, where that cluster does not fit (up to 16
+// blocks of 1,024 threads at once is more than a context limited to part of the
+// SMs may have) or the launch is refused: the caller then takes the sort of
+// several kernels.
 template <class Key, int R, class... Params, class... Args>
-inline cudaError_t launch_small_sort(void (*kernel)(Params...), uint32_t n, cudaStream_t st, Args... args) {
+inline bool launch_small_sort(void (*kernel)(Params...), uint32_t n, cudaStream_t st, Args... args) {
     constexpr int smem = small_sort_smem_bytes<Key, R>();
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = small_sort_blocks(n, R);
@@ -176,7 +178,13 @@ inline cudaError_t launch_small_sort(void (*kernel)(Params...), uint32_t n, cuda
     cfg.stream = st;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
+    int clusters = 0;
+    const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+                    cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0 &&
+                    cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok;
 }
 
 }  // namespace pm

@@ -49,7 +49,7 @@ def desc(**kw):
 
 
 def launched(log, name):
-    return [x for x in log if x.split()[0] in ("launch", "cluster") and x.split()[1].startswith(name)]
+    return [x for x in log if x.startswith(("launch " + name, "cluster " + name))]
 
 
 @pytest.fixture(scope="module")
@@ -118,3 +118,25 @@ def test_shared_walk_asks_for_its_block_size_once(engine, lists):
         asked.append(sum(x.startswith("occupancy k_knn_shared") for x in log))
     assert asked == [5, 0, 5, 0, 0]
     engine.lib.pm_destroy(h)
+
+
+@pytest.mark.parametrize("setting,value", [("clusters", 0), ("refuse_clusters", 1)])
+@pytest.mark.parametrize("n", [2, 16385, 32769, 65536])
+def test_small_sorts_without_room_for_a_cluster(engine, setting, value, n):
+    """Maps and query sets of up to 65,536 elements take the sorts of several
+    kernels where one cluster does not fit, or its launch is refused."""
+    several = ["k_bounds", "k_morton", "k_digit_scatter<unsigned long", "k_query_order", "k_digit_scatter<unsigned int"]
+    h = engine.map(n, n)
+    try:
+        for fits in (True, False):
+            engine.set(setting, value if not fits else {"clusters": 8, "refuse_clusters": 0}[setting])
+            engine.log()
+            assert engine.build(h, n) == L.PM_OK and engine.query(h, n) == L.PM_OK
+            log = engine.log()
+            assert len(launched(log, "k_small_build")) == len(launched(log, "k_small_query_sort")) == (1 if fits else 0)
+            assert [bool(launched(log, x)) for x in several] == [not fits] * len(several)
+            assert launched(log, "k_knn_group")
+    finally:
+        engine.set("clusters", 8)
+        engine.set("refuse_clusters", 0)
+        engine.lib.pm_destroy(h)
