@@ -1366,7 +1366,9 @@ pm_status batch_query_device(pm_batch* b, uint32_t kmax, const float* d_qpos4, c
     QueryOutputs out{reinterpret_cast<float4*>(d_rad4), d_nbr, d_r2, d_count};
     QueryTuning t = tuning_of(m);
     t.stats = nullptr;
-    if (t.layout == PM_KBUF_WIDE) {   // query records in processing order
+    if (t.layout == PM_KBUF_WIDE && shared_walk(b->total_photons, nq)) {
+        // query records in processing order, for the shared walk alone: a batch's
+        // single search reads through the order
         nl += gather_queries(vals[cur], qpos, reinterpret_cast<const float4*>(d_qnrm4), nq, P<float4>(m->qsorted), st);
         t.qsorted = P<float4>(m->qsorted);
     }

@@ -1640,7 +1640,7 @@ static uint32_t grid_for(K kernel, int threads, int smem, uint32_t rounds, int w
 //   1M photons:      k = 50: 503,316 1.29 / 1.26, 1,006,632 2.36 / 1.57;
 //                    k = 100: 503,316 1.65 / 1.87, 671,088 2.11 / 2.08, 1,006,632 3.02 / 2.22
 // The line follows the break-even points: 640 sqrt(photons), 262,144 at least.
-static bool shared_walk(uint32_t n, uint32_t nq) {
+bool shared_walk(uint32_t n, uint32_t nq) {
     return nq >= 262144u && (uint64_t)nq * nq >= 409600ull * n;
 }
 

@@ -140,3 +140,18 @@ def test_small_sorts_without_room_for_a_cluster(engine, setting, value, n):
         engine.set("clusters", 8)
         engine.set("refuse_clusters", 0)
         engine.lib.pm_destroy(h)
+
+
+@pytest.mark.parametrize("nq,shared", [(262143, False), (262144, True)])
+def test_batch_lays_records_out_for_the_shared_walk_only(engine, nq, shared):
+    b = C.c_void_p()
+    assert engine.lib.pm_batch_create(C.byref(b)) == L.PM_OK
+    photons, queries = (C.c_uint32 * 3)(0, 400, 1000), (C.c_uint32 * 3)(0, 7, nq)
+    descs = (L.QueryDesc * 2)(desc(), desc())
+    assert engine.lib.pm_batch_build(b, 16, 32, photons, 2, L.PM_PHOTONS_PACKED, None) == L.PM_OK
+    engine.log()
+    assert engine.lib.pm_batch_query(b, descs, 16, 32, queries, 48, None, None, None, None) == L.PM_OK
+    log = engine.log()
+    assert len(launched(log, "k_knn_shared<true")) == len(launched(log, "k_gather_queries")) == int(shared)
+    assert len(launched(log, "k_knn_group<32, false, true, true>")) == int(not shared)
+    assert engine.lib.pm_batch_destroy(b) == L.PM_OK
