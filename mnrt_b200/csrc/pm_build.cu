@@ -123,6 +123,7 @@ __global__ void __launch_bounds__(kBoundsThreads) k_bounds(const float4* __restr
     hdr->max_power = r[6];
     hdr->fix_scale = fix_scale_of(r[6]);
     hdr->n = n;
+    hdr->nonfinite = rb;
     if (rb) atomicOr(&hdr->errors, kErrNonFinite);
     *reinterpret_cast<unsigned int*>(partials + 8 * gridDim.x) = 0u;   // ready for the next build
 }
@@ -570,7 +571,8 @@ __global__ void __launch_bounds__(kSmallSortThreads, 1) k_small_build(const floa
         hdr->max_power = s_all[6];
         hdr->fix_scale = fix_scale_of(s_all[6]);
         hdr->n = n;
-        hdr->errors = __float_as_uint(s_all[7]) ? kErrNonFinite : 0u;
+        hdr->nonfinite = __float_as_uint(s_all[7]);
+        hdr->errors = hdr->nonfinite ? kErrNonFinite : 0u;
     }
     const float ext = fmaxf(fmaxf(__fsub_rn(s_all[3], s_all[0]), __fsub_rn(s_all[4], s_all[1])),
                             __fsub_rn(s_all[5], s_all[2]));

@@ -54,7 +54,7 @@ struct MapHeader {
     uint32_t n;
     uint32_t num_nodes; // internal nodes (excluding the super-root at index 0)
     uint32_t errors;
-    uint32_t pad;
+    uint32_t nonfinite; // a photon's position is not finite (kept when errors are cleared; single maps)
 };
 
 // ------------------------------------------------------------ arithmetic --

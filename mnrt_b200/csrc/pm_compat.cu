@@ -77,10 +77,8 @@ __device__ __forceinline__ void extent_of(const float* lo, const float* hi, floa
     rad = __fmul_rn(__fsqrt_rn(d2), 0.5f);
 }
 
-// Upper bound of d2_rn(q, p) over every p inside [lo, hi], rounded as d2_rn is
-// (infinite for a box with a non-finite side: such photons are tested one by one).
+// Upper bound of d2_rn(q, p) over every p inside [lo, hi], rounded as d2_rn is.
 __device__ __forceinline__ float box_ub(float qx, float qy, float qz, const float* lo, const float* hi) {
-    if (!isfinite((lo[0] + lo[1] + lo[2]) + (hi[0] + hi[1] + hi[2]))) return INFINITY;
     const float gx = fmaxf(fabsf(__fsub_rn(lo[0], qx)), fabsf(__fsub_rn(hi[0], qx)));
     const float gy = fmaxf(fabsf(__fsub_rn(lo[1], qy)), fabsf(__fsub_rn(hi[1], qy)));
     const float gz = fmaxf(fabsf(__fsub_rn(lo[2], qz)), fabsf(__fsub_rn(hi[2], qz)));
@@ -160,6 +158,10 @@ __device__ __forceinline__ bool warp_range(const MapView& m, float qx, float qy,
 __device__ float refine_radius(const MapView& m, float qx, float qy, float qz, float radius_max, uint32_t k,
                                uint32_t iters, CompatSmem& s, uint32_t lane, bool& ok) {
     float r_min = 0.0f, r_max = radius_max;
+    // A photon without a finite position is in range of nothing, and a leaf's box
+    // need not show it (the minima of a box drop a NaN): such a map's photons are
+    // tested one by one.
+    const bool one_by_one = m.hdr->nonfinite != 0;
     for (uint32_t it = 0; it < iters; ++it) {
         const float r = r_max, lo = r_min;
         const float delta = __fsub_rn(r_max, r_min);
@@ -173,7 +175,7 @@ __device__ float refine_radius(const MapView& m, float qx, float qy, float qz, f
         const float r2 = __fmul_rn(r, r);
         ok = warp_range(m, qx, qy, qz, r2, s, lane,
                         [&](float lb, float ub, uint32_t cnt) {
-                            if (!(ub < r2)) return false;
+                            if (one_by_one || !(ub < r2)) return false;
                             const uint32_t b = bin(lb);
                             if (b != bin(ub)) return false;
                             atomicAdd(&s.hist[b], cnt);

@@ -42,3 +42,27 @@ def test_compat_ranges(cuda, oracle_mod, n, nq, k, r, iters, filt):
     e = radiance_errors(out["rad"].cpu().numpy()[:, :3], o_rad)
     assert e["max"] <= 1e-5, format_errors(e)
     assert pm.info().device_errors == 0
+
+
+@pytest.mark.parametrize("leaf", [32, 64])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_compat_counts_finite_photons_only(cuda, leaf, bad):
+    """Photons without a finite position are in no range: radii, counts and r^2 are
+    those of the map of the other photons (a tree too small for node estimates,
+    so that a radius depends on the photons in range alone)."""
+    n, nq, kw = 4000, 2000, dict(k=50, r_max=0.6)
+    ph = gen.photons(n, seed=5, caustic_frac=0.5)
+    q = gen.queries(nq, seed=6)
+    good = np.arange(n) % 7 != 3
+    ph.pos[~good, 0] = bad
+    qp, qn = to_dev(q.pos, cuda), to_dev(q.nrm, cuda)
+    got = []
+    for keep in (np.ones(n, bool), good):
+        pm = PhotonMap(n, global_q_radius_max=0.6)
+        pm.set_tuning(leaf_size=leaf)
+        pm.build(to_dev(ph.pos[keep], cuda), to_dev(ph.pow[keep], cuda))
+        pm.clear_errors()   # the header's error bits may be cleared at any time
+        out = pm.query(qp, qn, mode=L.PM_MODE_ZHOU_COMPAT, filter="box", **kw)
+        got.append([pm.compute_query_radii(qp, **kw), out["count"], out["r2"]])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
