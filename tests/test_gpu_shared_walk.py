@@ -2,6 +2,9 @@
 (k_knn_shared); queries in the given order are searched one by one.  Every
 output of the two must have the same bits: the neighbour sets are exact and the
 flux sums do not depend on the order of their terms."""
+import ctypes as C
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -117,3 +120,61 @@ def test_shared_walk_in_a_batch(cuda):
                     assert torch.equal(o[name][s].view(torch.int32), one[name].view(torch.int32)), (i, name)
             assert torch.equal(lists["nbr"][at:at + m * ks[i]].view(m, ks[i]), one["nbr"]), i
         at += m * ks[i]
+
+
+@pytest.mark.parametrize("nbr", [False, True])
+def test_shared_walk_without_allocations(cuda, nbr):
+    """pm_query_noalloc at its largest size shares walks too, and reads the queries
+    through the order instead of from records."""
+    n, nq, k = 60000, L.PM_NOALLOC_MAX_QUERIES, 40
+    ph, q = gen.photons(n, seed=21, caustic_frac=0.2), gen.queries(nq, seed=22, cluster_frac=0.5)
+    pm = PhotonMap(n, global_q_radius_max=0.1)
+    pm.build(to_dev(ph.pos, cuda), to_dev(ph.pow, cuda))
+    qp, qn = to_dev(q.pos, cuda), to_dev(q.nrm, cuda)
+    want = pm.query(qp, qn, want_nbr=nbr, sorted_queries=False, k=k, filter="cone")
+    got = {name: torch.full_like(x, -1) for name, x in want.items()}
+    d = pm.desc(k=k, filter="cone")
+    lib = L.load()
+    st = lib.pm_query_noalloc(pm.handle, C.byref(d), qp.data_ptr(), qn.data_ptr(), nq, got["rad"].data_ptr(),
+                              got["nbr"].data_ptr() if nbr else None, got["r2"].data_ptr(), got["count"].data_ptr(),
+                              torch.cuda.current_stream().cuda_stream)
+    assert st == L.PM_OK
+    torch.cuda.synchronize()
+    for name in want:
+        assert torch.equal(got[name].view(torch.int32), want[name].view(torch.int32)), name
+
+
+def test_shared_walk_from_two_threads(cuda):
+    """Two maps queried by two host threads at once, with different k: handles are
+    independent, every call answers every query."""
+    n, nq = 20000, 262144
+    ph, q = gen.photons(n, seed=31), gen.queries(nq, seed=32)
+    arrays = [to_dev(a, cuda) for a in (ph.pos, ph.pow, q.pos, q.nrm)]
+    work = []
+    for k in (100, 128):
+        pm = PhotonMap(n, global_q_radius_max=0.1)
+        pm.build(*arrays[:2])
+        want = pm.query(*arrays[2:], sorted_queries=False, k=k, filter="box")
+        work.append((pm, k, want, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    wrong = []
+
+    def run(pm, k, want, stream):
+        out = {name: torch.empty_like(x) for name, x in want.items()}
+        for _ in range(50):
+            with torch.cuda.stream(stream):
+                for x in out.values():
+                    x.fill_(-1)
+                try:
+                    pm.query(*arrays[2:], out=out, k=k, filter="box")
+                except L.PMError as e:
+                    wrong.append(str(e))
+            stream.synchronize()
+            wrong.extend(name for name in out if not torch.equal(out[name].view(torch.int32), want[name].view(torch.int32)))
+
+    threads = [threading.Thread(target=run, args=w) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
