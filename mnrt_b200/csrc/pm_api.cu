@@ -45,7 +45,9 @@ struct pm_map {
     uint32_t cap_queries = 0;   // capacity of query-sized buffers
     // photon-sized
     DevBuf pos, pow, inv, nodes, hdr;
-    DevBuf keys0, keys1, vals0, vals1, scratch, kfirst, klast, ksplit, kkeep, krank, parent, arrive, nleaf, partials;
+    // the build's scratch in one block (build_buffers); between builds it holds
+    // the adjoint's photon records
+    DevBuf build_block, scratch, ksplit, kkeep, krank, parent, arrive, nleaf, partials;
     DevBuf wslot, wcnt, wfirst, wchild, wroot, wscan, rootmark;   // 32-wide tree
     // query-sized
     DevBuf qkeys0, qkeys1, qvals0, qvals1, qscratch, counter, fixq, qsorted;
@@ -53,7 +55,7 @@ struct pm_map {
     uint32_t shared_shapes[kSharedShapes] = {};   // QueryTuning::shared_shapes
     // backward (pm_query_backward): pair sort, per-query records, segments,
     // FP64 running sums, and the forward outputs when the kNN is recomputed
-    DevBuf bvals, bvals1, bkeys0, bkeys1, bscratch, blong, qrec, bphoton, seg_start, seg_end, acc;
+    DevBuf bvals, bvals1, bkeys0, bkeys1, bscratch, blong, qrec, seg_start, seg_end, acc;
     DevBuf rnbr, rcnt, rr2, rrad;
     DevBuf gnrm, gest;        // pm_gather_for: flipped normals, estimates
     // PM_MODE_ZHOU_COMPAT: node radius estimates of the current tree, kept
@@ -160,6 +162,13 @@ constexpr uint32_t kMaxQueries = 0x7fffffffu;
 
 size_t sort_words(uint32_t n) { return sort_scratch_words(n) + 1 + scan_scratch_words(n) + 64; }
 
+// Words of pm_map::build_block for cap photons: two key and two value arrays of
+// the sort and the radix tree's ranges, each of whole 256-byte lines; eight words
+// per photon, as many as a BwdPhoton has.
+size_t build_block_lane(size_t cap) { return (cap + 63) / 64 * 64; }
+size_t build_block_words(size_t cap) { return 8 * build_block_lane(cap); }
+static_assert(sizeof(BwdPhoton) == 8 * sizeof(uint32_t), "the records fit the build's scratch");
+
 pm_status ensure_photon_capacity(pm_map* m, uint32_t n, cudaStream_t st) {
     if (n <= m->cap_photons && m->hdr.ptr) return PM_OK;
     if (capturing(st))
@@ -172,13 +181,8 @@ pm_status ensure_photon_capacity(pm_map* m, uint32_t n, cudaStream_t st) {
     ENSURE(inv, cap * sizeof(uint32_t));
     ENSURE(nodes, (cap + 1) * sizeof(Node));
     ENSURE(hdr, sizeof(MapHeader));
-    ENSURE(keys0, cap * sizeof(uint64_t));
-    ENSURE(keys1, cap * sizeof(uint64_t));
-    ENSURE(vals0, cap * sizeof(uint32_t));
-    ENSURE(vals1, cap * sizeof(uint32_t));
+    ENSURE(build_block, build_block_words(cap) * sizeof(uint32_t) + 32);
     ENSURE(scratch, sort_words((uint32_t)cap) * sizeof(uint32_t));
-    ENSURE(kfirst, cap * sizeof(uint32_t));
-    ENSURE(klast, cap * sizeof(uint32_t));
     ENSURE(ksplit, cap * sizeof(uint32_t));
     ENSURE(kkeep, cap * sizeof(uint32_t));
     ENSURE(krank, cap * sizeof(uint32_t));
@@ -237,6 +241,20 @@ pm_status validate_desc(pm_map* m, const pm_query_desc* d, bool exact_only, bool
     if (d->order != PM_ORDER_SORTED && d->order != PM_ORDER_AS_GIVEN)
         return fail(m, PM_ERR_INVALID, "unknown query order %d", d->order);
     return PM_OK;
+}
+
+BuildBuffers build_buffers(pm_map* m) {
+    BuildBuffers bb;
+    const size_t lane = build_block_lane(m->cap_photons);
+    uint32_t* w = align32<uint32_t>(m->build_block);
+    bb.keys[0] = reinterpret_cast<uint64_t*>(w); bb.keys[1] = reinterpret_cast<uint64_t*>(w + 2 * lane);
+    bb.vals[0] = w + 4 * lane; bb.vals[1] = w + 5 * lane;
+    bb.kfirst = w + 6 * lane; bb.klast = w + 7 * lane;
+    bb.scratch = P<uint32_t>(m->scratch); bb.ksplit = P<uint32_t>(m->ksplit);
+    bb.kkeep = P<uint32_t>(m->kkeep); bb.krank = P<uint32_t>(m->krank);
+    bb.parent = P<uint32_t>(m->parent); bb.arrive = P<uint32_t>(m->arrive); bb.nleaf = P<uint32_t>(m->nleaf);
+    bb.partials = P<uint32_t>(m->partials); bb.num_partials = 1184;
+    return bb;
 }
 
 MapView view_of(pm_map* m) {
@@ -330,12 +348,11 @@ pm_status pm_create(pm_map** out, uint32_t max_photons, const float* aabb_min, c
 
 pm_status pm_destroy(pm_map* m) {
     if (!m) return PM_ERR_INVALID;
-    DevBuf* all[] = {&m->pos, &m->pow, &m->inv, &m->nodes, &m->hdr, &m->keys0, &m->keys1, &m->vals0, &m->vals1,
-                     &m->scratch, &m->kfirst, &m->klast, &m->ksplit, &m->kkeep, &m->krank, &m->parent,
+    DevBuf* all[] = {&m->pos, &m->pow, &m->inv, &m->nodes, &m->hdr, &m->build_block, &m->scratch, &m->ksplit, &m->kkeep, &m->krank, &m->parent,
                      &m->arrive, &m->nleaf, &m->partials, &m->wslot, &m->wcnt, &m->wfirst,
                      &m->wchild, &m->wroot, &m->wscan, &m->rootmark, &m->qkeys0, &m->qkeys1, &m->qvals0, &m->qvals1,
                      &m->qscratch, &m->counter, &m->fixq, &m->qsorted, &m->stats, &m->bvals, &m->bvals1, &m->bkeys0, &m->bkeys1, &m->blong,
-                     &m->bscratch, &m->qrec, &m->bphoton, &m->seg_start, &m->seg_end, &m->acc, &m->rnbr,
+                     &m->bscratch, &m->qrec, &m->seg_start, &m->seg_end, &m->acc, &m->rnbr,
                      &m->rcnt, &m->rr2, &m->rrad, &m->gnrm, &m->gest, &m->compat_est, &m->mpos, &m->mpow, &m->mflags,
                      &m->mrank, &m->mscan, &m->ic_pslot, &m->ic_level, &m->ic_range, &m->ic_center,
                      &m->ic_normal, &m->ic_est, &m->ic_exact, &m->ic_coarse, &m->ic_fin, &m->ic_work0, &m->ic_work1,
@@ -400,14 +417,7 @@ pm_status pm_build(pm_map* m, const float* d_pos4, const float* d_pow4, uint32_t
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     pm_status s = ensure_photon_capacity(m, n, st);
     if (s != PM_OK) return s;
-    BuildBuffers bb;
-    bb.keys[0] = P<uint64_t>(m->keys0); bb.keys[1] = P<uint64_t>(m->keys1);
-    bb.vals[0] = P<uint32_t>(m->vals0); bb.vals[1] = P<uint32_t>(m->vals1);
-    bb.scratch = P<uint32_t>(m->scratch);
-    bb.kfirst = P<uint32_t>(m->kfirst); bb.klast = P<uint32_t>(m->klast); bb.ksplit = P<uint32_t>(m->ksplit);
-    bb.kkeep = P<uint32_t>(m->kkeep); bb.krank = P<uint32_t>(m->krank);
-    bb.parent = P<uint32_t>(m->parent); bb.arrive = P<uint32_t>(m->arrive); bb.nleaf = P<uint32_t>(m->nleaf);
-    bb.partials = P<uint32_t>(m->partials); bb.num_partials = 1184;
+    const BuildBuffers bb = build_buffers(m);
     const bool prof = m->profiling && !capturing(st);
     if (prof) cudaEventRecord(m->ev[0], st);
     const int nl = build_map(reinterpret_cast<const float4*>(d_pos4), reinterpret_cast<const float4*>(d_pow4), n,
@@ -653,7 +663,6 @@ static pm_status ensure_bwd_capacity(pm_map* m, uint32_t chunk_q, uint32_t k, bo
     ENSURE(blong, ((size_t)n + 1) * sizeof(uint32_t));
     // 32-byte loads, and a caller's allocator may align to 16 only
     ENSURE(qrec, qc * sizeof(BwdQuery) + 32);
-    ENSURE(bphoton, (size_t)n * sizeof(BwdPhoton) + 32);
     ENSURE(seg_start, (size_t)n * sizeof(uint32_t));
     ENSURE(seg_end, (size_t)n * sizeof(uint32_t));
     if (chunked) ENSURE(acc, (size_t)n * 6 * sizeof(double));
@@ -713,7 +722,8 @@ pm_status pm_query_backward(pm_map* m, const pm_query_desc* desc, const float* d
     a.cone_k = desc->filter == PM_FILTER_CONE ? desc->cone_k : 1.0f;
     a.min_found = desc->min_found;
     a.qrec = align32<BwdQuery>(m->qrec);
-    a.photon = align32<BwdPhoton>(m->bphoton);
+    BwdPhoton* const photons = align32<BwdPhoton>(m->build_block);   // idle between builds
+    a.photon = photons;
     a.vals = nullptr; a.cursor = nullptr; a.pair_cap = 0;
     a.nbr = nullptr; a.count_in = nullptr; a.order = nullptr;
     BwdBuffers b;
@@ -723,7 +733,7 @@ pm_status pm_query_backward(pm_map* m, const pm_query_desc* desc, const float* d
     b.seg_start = P<uint32_t>(m->seg_start); b.seg_end = P<uint32_t>(m->seg_end);
     b.long_count = P<uint32_t>(m->blong); b.long_list = b.long_count + 1;
     b.acc = P<double>(m->acc);
-    int nl = bwd_pack(a.pos, a.pow, m->n, align32<BwdPhoton>(m->bphoton), st);
+    int nl = bwd_pack(a.pos, a.pow, m->n, photons, st);
     for (uint32_t c = 0; c < nchunks; ++c) {
         const uint32_t q0 = c * chunk;
         const uint32_t nqc = nq ? ((nq - q0) < chunk ? (nq - q0) : chunk) : 0;
@@ -1321,14 +1331,7 @@ pm_status batch_upload_queries(pm_batch* b, const pm_query_desc* descs, const ui
 pm_status batch_build_device(pm_batch* b, const float* d_pos4, const float* d_pow4, int format, cudaStream_t st) {
     pm_map* m = b->m;
     const uint32_t n = b->total_photons, maps = b->num_maps;
-    BuildBuffers bb;
-    bb.keys[0] = P<uint64_t>(m->keys0); bb.keys[1] = P<uint64_t>(m->keys1);
-    bb.vals[0] = P<uint32_t>(m->vals0); bb.vals[1] = P<uint32_t>(m->vals1);
-    bb.scratch = P<uint32_t>(m->scratch);
-    bb.kfirst = P<uint32_t>(m->kfirst); bb.klast = P<uint32_t>(m->klast); bb.ksplit = P<uint32_t>(m->ksplit);
-    bb.kkeep = P<uint32_t>(m->kkeep); bb.krank = P<uint32_t>(m->krank);
-    bb.parent = P<uint32_t>(m->parent); bb.arrive = P<uint32_t>(m->arrive); bb.nleaf = P<uint32_t>(m->nleaf);
-    bb.partials = P<uint32_t>(m->partials); bb.num_partials = 1184;
+    const BuildBuffers bb = build_buffers(m);
     const float4* pos = reinterpret_cast<const float4*>(d_pos4);
     const float4* pw = reinterpret_cast<const float4*>(d_pow4);
     int nl = batch_bounds_and_keys(pos, pw, P<uint32_t>(b->ph_off), maps, n, P<uint32_t>(b->acc),

@@ -81,11 +81,10 @@ void __cudaRegisterFunction(void**, const char* fun, char*, const char* name, in
     char* plain = abi::__cxa_demangle(name, nullptr, nullptr, &status);
     std::string s = status == 0 ? plain : name;
     std::free(plain);
-    const size_t args = s.find('(');   // "void pm::k_name<...>(...)" -> "k_name<...>"
-    s = s.substr(0, args);
+    // "void pm::(anonymous namespace)::k_name<...>(...)" -> "k_name<...>"
     const size_t k = s.find("k_");
     std::lock_guard<std::mutex> l(g_mu);
-    g_names[fun] = k == std::string::npos ? s : s.substr(k);
+    g_names[fun] = k == std::string::npos ? s : s.substr(k, s.find('(', k) - k);
 }
 unsigned __cudaPushCallConfiguration(dim3 grid, dim3 block, size_t smem, void* stream) {
     t_config = {grid, block, smem, static_cast<cudaStream_t>(stream)};

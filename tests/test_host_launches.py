@@ -155,3 +155,18 @@ def test_batch_lays_records_out_for_the_shared_walk_only(engine, nq, shared):
     assert len(launched(log, "k_knn_shared<true")) == len(launched(log, "k_gather_queries")) == int(shared)
     assert len(launched(log, "k_knn_group<32, false, true, true>")) == int(not shared)
     assert engine.lib.pm_batch_destroy(b) == L.PM_OK
+
+
+def test_first_adjoint_takes_no_storage_for_photon_records(engine):
+    """The adjoint's 32-byte photon records lie in the build's scratch, which is idle
+    between builds: a map's first adjoint allocates four bytes a photon an array."""
+    n, nq = 100000, 10
+    h = engine.map(n, nq)
+    assert engine.build(h, n) == L.PM_OK
+    engine.log()
+    assert engine.lib.pm_query_backward(h, C.byref(desc(k=1)), 16, 32, nq, 48, 64, None, 80, 96, 112, None) == L.PM_OK
+    log = engine.log()
+    sizes = [int(x.split()[1]) for x in log if x.startswith("malloc")]
+    assert len(sizes) == 6 and max(sizes) <= 4 * (n + 1)
+    assert launched(log, "k_bwd_prep")
+    engine.lib.pm_destroy(h)
