@@ -723,7 +723,7 @@ pm_status pm_query_backward(pm_map* m, const pm_query_desc* desc, const float* d
     a.min_found = desc->min_found;
     a.qrec = align32<BwdQuery>(m->qrec);
     BwdPhoton* const photons = align32<BwdPhoton>(m->build_block);   // idle between builds
-    a.photon = photons;
+    a.photon = bwd_packs((uint64_t)nq * k, m->n) ? photons : nullptr;
     a.vals = nullptr; a.cursor = nullptr; a.pair_cap = 0;
     a.nbr = nullptr; a.count_in = nullptr; a.order = nullptr;
     BwdBuffers b;
@@ -733,7 +733,7 @@ pm_status pm_query_backward(pm_map* m, const pm_query_desc* desc, const float* d
     b.seg_start = P<uint32_t>(m->seg_start); b.seg_end = P<uint32_t>(m->seg_end);
     b.long_count = P<uint32_t>(m->blong); b.long_list = b.long_count + 1;
     b.acc = P<double>(m->acc);
-    int nl = bwd_pack(a.pos, a.pow, m->n, photons, st);
+    int nl = a.photon ? bwd_pack(a.pos, a.pow, m->n, photons, st) : 0;
     for (uint32_t c = 0; c < nchunks; ++c) {
         const uint32_t q0 = c * chunk;
         const uint32_t nqc = nq ? ((nq - q0) < chunk ? (nq - q0) : chunk) : 0;

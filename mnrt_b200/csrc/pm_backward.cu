@@ -97,6 +97,16 @@ __device__ __forceinline__ BwdPhoton load_photon(const BwdPhoton* p) {
                      __uint_as_float(v[4]), __uint_as_float(v[5]), __uint_as_float(v[6]), v[7]};
 }
 
+// The photon a neighbour list names: its record (kPacked), or position and flux
+// through the inverse permutation.
+template <bool kPacked>
+__device__ __forceinline__ BwdPhoton bwd_photon(const BwdArgs& a, uint32_t caller) {
+    if constexpr (kPacked) return load_photon(a.photon + caller);
+    const uint32_t t = a.inv[caller];
+    const float4 p = a.pos[t], w = a.pow[t];
+    return BwdPhoton{p.x, p.y, p.z, t, w.x, w.y, w.z, __float_as_uint(w.w)};
+}
+
 __device__ __forceinline__ BwdQuery load_query(const BwdQuery* p) {
     uint32_t v[8], w[8];
     ld_record32(p, v);
@@ -156,6 +166,7 @@ __device__ __forceinline__ uint32_t bwd_found(const BwdArgs& a, uint32_t ql, uin
 // filter reciprocal), decided without the query's position or r^2.
 __device__ __forceinline__ bool bwd_placed(const BwdArgs& a, uint32_t cnt) { return cnt > 0 && cnt >= a.min_found; }
 
+template <bool kPacked>
 __device__ __forceinline__ BwdHead bwd_head(const BwdArgs& a, uint32_t ql, uint32_t q, uint32_t lane) {
     const uint32_t k = a.k;
     const uint32_t* row = a.nbr + (size_t)ql * k;
@@ -163,7 +174,7 @@ __device__ __forceinline__ BwdHead bwd_head(const BwdArgs& a, uint32_t ql, uint3
     h.cnt = bwd_found(a, ql, lane);
     h.qp = a.qpos[q];
     h.r2 = (double)a.r_max * (double)a.r_max;
-    if (h.cnt == k) h.r2 = dist2_d(load_photon(a.photon + row[k - 1]), h.qp);
+    if (h.cnt == k) h.r2 = dist2_d(bwd_photon<kPacked>(a, row[k - 1]), h.qp);
     h.active = h.cnt > 0 && h.cnt >= a.min_found && h.r2 > 0.0 && isfinite(h.qp.x) && isfinite(h.qp.y) &&
                isfinite(h.qp.z);
     return h;
@@ -214,7 +225,7 @@ __global__ void __launch_bounds__(256) k_bwd_count(BwdArgs a, uint32_t q0, uint3
 // Five blocks per SM (48 registers, a few spilled): 40 warps hide the
 // dependent gathers better than 32 at 64 registers (1M x 1M, k = 64: adjoint
 // 2.98 -> 2.88 ms).
-template <bool kPlace>
+template <bool kPlace, bool kPacked>
 __global__ void __launch_bounds__(256, 5) k_bwd_prep(BwdArgs a, uint32_t q0, uint32_t nq_chunk) {
     const uint32_t warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t lane = threadIdx.x & 31u;
@@ -222,7 +233,7 @@ __global__ void __launch_bounds__(256, 5) k_bwd_prep(BwdArgs a, uint32_t q0, uin
     const uint32_t ql = a.order ? a.order[warp_global] : warp_global, q = q0 + ql;
     const uint32_t k = a.k;
     const uint32_t* row = a.nbr + (size_t)ql * k;
-    const BwdHead h = bwd_head(a, ql, q, lane);
+    const BwdHead h = bwd_head<kPacked>(a, ql, q, lane);
     const float4 qp = h.qp;
     const float4 qn = a.qnrm[q];
     const double r2 = h.r2;
@@ -239,7 +250,7 @@ __global__ void __launch_bounds__(256, 5) k_bwd_prep(BwdArgs a, uint32_t q0, uin
             a.vals[pair0 + j] = val;
             continue;
         }
-        const BwdPhoton pp = load_photon(a.photon + row[j]);
+        const BwdPhoton pp = bwd_photon<kPacked>(a, row[j]);
         const uint32_t slot = kPlace ? atomicAdd(&a.cursor[pp.tree], 1u) : 0u;
         if (active && front_rn(qn.x, qn.y, qn.z, pp.dir)) {
             double w, dwd, dwr;
@@ -518,7 +529,7 @@ int backward_chunk(const BwdArgs& a, uint32_t q0, uint32_t nq_chunk, bool first,
         x.keys = b.keys[0];
         x.vals = b.vals[0];
         x.cursor = nullptr;
-        k_bwd_prep<false><<<qblocks, 32 * warps_per_block, 0, st>>>(x, q0, nq_chunk);
+        k_bwd_prep<false, true><<<qblocks, 32 * warps_per_block, 0, st>>>(x, q0, nq_chunk);   // so many pairs are packed
         ++nl;
         uint32_t* keys[2] = {b.keys[0], b.keys[1]};
         uint32_t* vals[2] = {b.vals[0], b.vals[1]};
@@ -541,7 +552,8 @@ int backward_chunk(const BwdArgs& a, uint32_t q0, uint32_t nq_chunk, bool first,
         nl += exclusive_scan(b.seg_end, b.seg_end, a.n, b.scratch, nullptr, st);
         cudaMemcpyAsync(b.seg_start, b.seg_end, (size_t)a.n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
         if (nq_chunk > 0) {
-            k_bwd_prep<true><<<qblocks, 32 * warps_per_block, 0, st>>>(x, q0, nq_chunk);
+            if (x.photon) k_bwd_prep<true, true><<<qblocks, 32 * warps_per_block, 0, st>>>(x, q0, nq_chunk);
+            else k_bwd_prep<true, false><<<qblocks, 32 * warps_per_block, 0, st>>>(x, q0, nq_chunk);
             cudaMemsetAsync(b.long_count, 0, sizeof(uint32_t), st);
             k_bwd_segsort<<<(a.n + warps_per_block - 1) / warps_per_block, 32 * warps_per_block, 0, st>>>(
                 b.seg_start, b.seg_end, a.n, x.pair_cap, b.vals[0], b.long_list, b.long_count);

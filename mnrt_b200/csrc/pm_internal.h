@@ -284,7 +284,7 @@ struct __align__(32) BwdPhoton {
 static_assert(sizeof(BwdPhoton) == 32, "one 32-byte record per photon");
 
 struct BwdArgs {
-    const BwdPhoton* photon;  // caller order (bwd_pack)
+    const BwdPhoton* photon;  // caller order (bwd_pack), or nullptr: too few pairs to pay for them
     const float4* pos;        // tree order
     const float4* pow;
     const uint32_t* inv;      // caller index -> tree position
@@ -319,6 +319,13 @@ struct BwdBuffers {
 // radix sort instead of counts, atomic placement and segment sorts.
 constexpr uint64_t kBwdPlaceMaxFanIn = 256;
 inline bool bwd_sort_path(uint64_t pairs, uint32_t n) { return pairs > kBwdPlaceMaxFanIn * (uint64_t)n; }
+// Pairs per photon from which the photons' records are laid out first (bwd_pack): the
+// layout costs every photon 64 bytes, and saves a pair two of its gathers.  Adjoint
+// without / with records, us: 1M photons, 0.1 pairs each 144 / 179, 8 each (k = 64)
+// 539 / 540, 32 each 1,398 / 1,363, 64 each 2,677 / 2,602; 8M photons, 0.1 each 1,366 /
+// 1,556, 8 each 3,910 / 3,987; 65,536 photons, 16 each 102 / 105, 250 each 1,905 / 1,890.
+constexpr uint64_t kBwdPackMin = 32;
+inline bool bwd_packs(uint64_t pairs, uint32_t n) { return pairs >= kBwdPackMin * (uint64_t)n; }
 size_t bwd_scratch_words(uint32_t n, uint64_t pairs, bool sort_path);
 int bwd_pack(const float4* pos, const float4* pow, uint32_t n, BwdPhoton* out, cudaStream_t st);
 int backward_chunk(const BwdArgs& a, uint32_t q0, uint32_t nq_chunk, bool first, bool last, const BwdBuffers& b,

@@ -180,3 +180,16 @@ def test_autograd_wrapper(cuda, oracle_mod):
                                       "epanechnikov")
     assert rel_err(pw.grad.cpu().numpy()[:, :3], hp, 1e-6).max() <= RTOL_HOST
     assert rel_err(pos.grad.cpu().numpy()[:, :3], hx, 1e-6).max() <= RTOL_HOST
+
+
+@pytest.mark.parametrize("nq,k", [(1, 8), (3999, 32), (4000, 32)])
+def test_backward_at_the_line_of_the_photon_records(cuda, oracle_mod, nq, k):
+    """Photon records in caller order are laid out from 32 pairs a photon up; below, the
+    per-query pass gathers through the inverse permutation.  RTOL_HOST on both sides."""
+    n, r, filt = 4000, 0.1, "cone"
+    ph, q, t, idx, cnt = setup_problem(oracle_mod, n, nq, k, r, filt, seed=90)
+    res = engine_grads(cuda, ph, q, t, k, r, filt)
+    hp, hx = oracle_mod.backward_fp64(ph.pos, ph.pow, q.pos, q.nrm, idx, cnt, k, r, res["g"][:, :3].astype(np.float64),
+                                      filt)
+    assert rel_err(res["gpow"][:, :3], hp, 1e-6).max() <= RTOL_HOST
+    assert rel_err(res["gpos"][:, :3], hx, 1e-6).max() <= RTOL_HOST

@@ -157,6 +157,21 @@ def test_batch_lays_records_out_for_the_shared_walk_only(engine, nq, shared):
     assert engine.lib.pm_batch_destroy(b) == L.PM_OK
 
 
+@pytest.mark.parametrize("nq,k,records", [(1, 8, False), (15999, 2, False), (16000, 2, True), (300, 128, True)])
+def test_adjoint_lays_photon_records_out_for_many_pairs_only(engine, nq, k, records):
+    """The records cost every photon: below 32 pairs a photon the adjoint gathers
+    through the inverse permutation."""
+    n = 1000
+    h = engine.map(n, nq)
+    assert engine.build(h, n) == L.PM_OK
+    engine.log()
+    assert engine.lib.pm_query_backward(h, C.byref(desc(k=k)), 16, 32, nq, 48, 64, None, 80, 96, 112, None) == L.PM_OK
+    log = engine.log()
+    assert len(launched(log, "k_bwd_pack")) == len(launched(log, "k_bwd_prep<true, true>")) == int(records)
+    assert len(launched(log, "k_bwd_prep<true, false>")) == int(not records)
+    engine.lib.pm_destroy(h)
+
+
 def test_first_adjoint_takes_no_storage_for_photon_records(engine):
     """The adjoint's 32-byte photon records lie in the build's scratch, which is idle
     between builds: a map's first adjoint allocates four bytes a photon an array."""
