@@ -107,7 +107,9 @@ __device__ __forceinline__ BwdPhoton bwd_photon(const BwdArgs& a, uint32_t calle
     return BwdPhoton{p.x, p.y, p.z, t, w.x, w.y, w.z, __float_as_uint(w.w)};
 }
 
+template <bool kWide>   // by two 256-bit loads, or four of 128 bits
 __device__ __forceinline__ BwdQuery load_query(const BwdQuery* p) {
+    if constexpr (!kWide) return *p;
     uint32_t v[8], w[8];
     ld_record32(p, v);
     ld_record32(reinterpret_cast<const unsigned char*>(p) + 32, w);
@@ -185,7 +187,8 @@ __device__ __forceinline__ BwdHead bwd_head(const BwdArgs& a, uint32_t ql, uint3
 // of the inverse permutation, the position and the flux.  A gather's cost is
 // the L1 lines it touches, once per load: 1.47 -> 1.26 ms for that pass (cold;
 // 1M x 1M, k = 64), and 0.71 -> 0.54 ms for the per-photon pass, whose 64-byte
-// query records take two such loads instead of four.
+// query records take two such loads instead of four.  Laid out from kBwdPackMin
+// pairs a photon up.
 __global__ void k_bwd_pack(const float4* __restrict__ pos, const float4* __restrict__ pw, uint32_t n,
                            BwdPhoton* __restrict__ out) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -443,6 +446,13 @@ int key_bits_for(uint32_t n) {
 
 // One thread per photon (tree position).  acc holds 6 doubles per photon
 // between chunks.
+// kWide: two 256-bit loads a record touch fewer L1 lines, which bounds the pass when
+// many warps gather; with few (a thread a photon: 157 blocks at 20,000 photons) the
+// chain of one photon's entries bounds it, and four 128-bit loads answer sooner.
+// Adjoint with 256-bit / 128-bit loads, us: 1,000 photons, 2,400 pairs each 693 / 643;
+// 20,000, 64 each (k = 8) 291 / 279; 65,536, 64 each 661 / 672; 1M, 64 each 2,602 / 2,702.
+constexpr uint32_t kReduceWideMin = 40000;
+template <bool kWide>
 __global__ void k_bwd_reduce(BwdArgs a, uint32_t q0, const uint32_t* __restrict__ sorted_vals,
                              const uint32_t* __restrict__ start, const uint32_t* __restrict__ end, int first, int last,
                              double* __restrict__ acc, float4* __restrict__ grad_pow, float4* __restrict__ grad_pos) {
@@ -460,14 +470,14 @@ __global__ void k_bwd_reduce(BwdArgs a, uint32_t q0, const uint32_t* __restrict_
         // software pipeline: the next entry's record and the value after it
         // load while this entry's math runs (the sums keep their order)
         uint32_t vnext = sorted_vals[b];   // query << 1 | (the photon is the query's k-th)
-        BwdQuery rnext = load_query(a.qrec + (vnext >> 1));
+        BwdQuery rnext = load_query<kWide>(a.qrec + (vnext >> 1));
         uint32_t vafter = b + 1 < e ? sorted_vals[b + 1] : 0u;
         for (uint32_t i = b; i < e; ++i) {
             const uint32_t v = vnext;
             const BwdQuery rec = rnext;
             if (i + 1 < e) {
                 vnext = vafter;
-                rnext = load_query(a.qrec + (vafter >> 1));
+                rnext = load_query<kWide>(a.qrec + (vafter >> 1));
                 vafter = i + 2 < e ? sorted_vals[i + 2] : 0u;
             }
             const double rinv = rec.rinv;
@@ -563,8 +573,9 @@ int backward_chunk(const BwdArgs& a, uint32_t q0, uint32_t nq_chunk, bool first,
         }
     }
     if (a.n > 0) {
-        k_bwd_reduce<<<(a.n + 127) / 128, 128, 0, st>>>(x, q0, sorted_vals, b.seg_start, b.seg_end, first ? 1 : 0,
-                                                        last ? 1 : 0, b.acc, grad_pow, grad_pos);
+        auto reduce = a.n >= kReduceWideMin ? k_bwd_reduce<true> : k_bwd_reduce<false>;
+        reduce<<<(a.n + 127) / 128, 128, 0, st>>>(x, q0, sorted_vals, b.seg_start, b.seg_end, first ? 1 : 0,
+                                                  last ? 1 : 0, b.acc, grad_pow, grad_pos);
         ++nl;
     }
     return nl;

@@ -172,6 +172,16 @@ def test_adjoint_lays_photon_records_out_for_many_pairs_only(engine, nq, k, reco
     engine.lib.pm_destroy(h)
 
 
+@pytest.mark.parametrize("n,wide", [(39999, False), (40000, True)])
+def test_adjoint_reduces_few_photons_by_short_loads(engine, n, wide):
+    h = engine.map(n, 100)
+    assert engine.build(h, n) == L.PM_OK
+    engine.log()
+    assert engine.lib.pm_query_backward(h, C.byref(desc(k=8)), 16, 32, 100, 48, 64, None, 80, 96, 112, None) == L.PM_OK
+    assert len(launched(engine.log(), f"k_bwd_reduce<{str(wide).lower()}>")) == 1
+    engine.lib.pm_destroy(h)
+
+
 def test_first_adjoint_takes_no_storage_for_photon_records(engine):
     """The adjoint's 32-byte photon records lie in the build's scratch, which is idle
     between builds: a map's first adjoint allocates four bytes a photon an array."""
