@@ -1247,6 +1247,7 @@ struct pm_batch {
     DevBuf ph_off, q_off, bq, geom, acc;
     uint32_t cap_maps = 0;
     std::vector<uint32_t> h_ph_off;   // host copy of the built photon offsets
+    bool shared[2] = {false, false};  // the uploaded queries share walks: without, with neighbour lists
     // CUDA graph of build + query
     cudaStream_t cap_stream = nullptr;
     cudaGraph_t graph = nullptr;
@@ -1299,6 +1300,7 @@ pm_status batch_upload_queries(pm_batch* b, const pm_query_desc* descs, const ui
     std::vector<BatchQuery> t(maps);
     uint32_t kmax = 1;
     uint64_t nbr = 0;
+    double gain[2] = {0.0, 0.0}, tail = 0.0;
     for (uint32_t i = 0; i < maps; ++i) {
         pm_status s = validate_desc(b->m, &descs[i], true);
         if (s != PM_OK) return s;
@@ -1318,7 +1320,12 @@ pm_status batch_upload_queries(pm_batch* b, const pm_query_desc* descs, const ui
         q.norm_c = filter_norm_const(q.filter, q.cone_k);
         nbr += (uint64_t)q.q_n * q.k;
         kmax = q.k > kmax ? q.k : kmax;
+        if (q.ph_n >= 1000 && q.q_n > 0) {   // smaller maps cost about the same either way
+            for (int l = 0; l < 2; ++l) gain[l] += shared_gain(q.ph_n, q.q_n, q.k, l == 1);
+            tail = std::max(tail, shared_tail(q.ph_n, q.k));
+        }
     }
+    for (int l = 0; l < 2; ++l) b->shared[l] = tail > 0.0 && shared_walk(offsets[maps], gain[l], tail);
     if (cudaMemcpy(b->bq.ptr, t.data(), maps * sizeof(BatchQuery), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(b->q_off.ptr, offsets, (maps + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice) != cudaSuccess)
         return check_cuda(b->m, "batch query tables");
@@ -1369,15 +1376,13 @@ pm_status batch_query_device(pm_batch* b, uint32_t kmax, const float* d_qpos4, c
     QueryOutputs out{reinterpret_cast<float4*>(d_rad4), d_nbr, d_r2, d_count};
     QueryTuning t = tuning_of(m);
     t.stats = nullptr;
-    if (t.layout == PM_KBUF_WIDE && shared_walk(b->total_photons, nq)) {
+    if (t.layout == PM_KBUF_WIDE && b->shared[d_nbr != nullptr]) {
         // query records in processing order, for the shared walk alone: a batch's
         // single search reads through the order
         nl += gather_queries(vals[cur], qpos, reinterpret_cast<const float4*>(d_qnrm4), nq, P<float4>(m->qsorted), st);
         t.qsorted = P<float4>(m->qsorted);
     }
-    MapView v = view_of(m);
-    v.n = b->total_photons;
-    nl += query_knn_batch(v, P<BatchQuery>(b->bq), P<BatchGeom>(b->geom), kmax, qpos,
+    nl += query_knn_batch(view_of(m), P<BatchQuery>(b->bq), P<BatchGeom>(b->geom), kmax, qpos,
                           reinterpret_cast<const float4*>(d_qnrm4), vals[cur], keys[cur], nq, out, P<uint32_t>(m->counter),
                           P<uint32_t>(m->fixq), reinterpret_cast<float*>(keys[cur ^ 1]), t, st);
     m->launches += (uint64_t)nl;

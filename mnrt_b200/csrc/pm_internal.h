@@ -182,10 +182,14 @@ struct QueryTuning {
     unsigned long long* stats;   // 8 traversal counters (group layout), nullptr = off
     uint32_t* shared_shapes;     // the handle's launch shapes of the shared walk (kSharedShapes words, 0: not asked yet)
     const float4* qsorted = nullptr;   // query records in sorted order (pos.xyz | caller index, normal), or nullptr
+                                       // (a batch: set where it shares walks)
 };
-// Whether sorted queries in the wide layout share walks (k_knn_shared): n photons, nq
-// queries, over all maps of a batch.
-bool shared_walk(uint32_t n, uint32_t nq);
+// Whether sorted queries in the wide layout share walks (k_knn_shared): nq of them in
+// all, the sum of what their maps gain (in queries, negative where one by one is
+// faster) and the largest of what their longest warps cost.
+double shared_gain(uint32_t n, uint32_t nq, uint32_t k, bool lists);
+double shared_tail(uint32_t n, uint32_t k);
+bool shared_walk(uint64_t nq, double gain, double tail);
 int gather_queries(const uint32_t* order, const float4* qpos, const float4* qnrm, uint32_t nq, float4* out, cudaStream_t st);
 int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const float4* qnrm,
               const uint32_t* order, uint32_t nq, const QueryOutputs& out, uint32_t* work_counter, uint32_t* fix_list, float* fix_bound,

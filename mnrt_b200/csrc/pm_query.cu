@@ -29,6 +29,7 @@
 #include "pm_internal.h"
 #include "pm_sort_small.cuh"
 #include <algorithm>
+#include <cmath>
 
 namespace pm {
 
@@ -1630,19 +1631,32 @@ static uint32_t grid_for(K kernel, int threads, int smem, uint32_t rounds, int w
 }
 
 // Whether enough queries are at hand to share walks (k_knn_shared).  Eight
-// queries cost less together, but a launch's longest warp takes longer (a chunk
-// in a dense blob: 0.3 ms with 65,536 photons, 0.9 with 1M), and sparse queries
-// reach more photons than fit.  One by one / shared, ms (R = 0.1, cone):
-//   65,536 photons:  k = 16: 131,072 queries 0.31 / 0.34, 262,144 0.52 / 0.42;
-//                    k = 100: 62,914 0.29 / 0.40
-//   300,001 photons: k = 16: 300,001 0.64 / 0.70, 450,001 0.90 / 0.75;
-//                    k = 100: 144,000 0.56 / 0.84, 288,000 0.95 / 0.95
-//   1M photons:      k = 50: 503,316 1.29 / 1.26, 1,006,632 2.36 / 1.57;
-//                    k = 100: 503,316 1.65 / 1.87, 671,088 2.11 / 2.08, 1,006,632 3.02 / 2.22
-// The line follows the break-even points: 640 sqrt(photons), 262,144 at least.
-bool shared_walk(uint32_t n, uint32_t nq) {
-    return nq >= 262144u && (uint64_t)nq * nq >= 409600ull * n;
+// neighbours of the curve must lie within their radii, which takes d(k) queries a
+// photon; with fewer a group is cut short and walks for one or two.  And a launch's
+// longest warp (a chunk in a dense blob) takes longer: t(n, k) queries more have to
+// pay for it.  Shared / one by one, the search alone (photons on walls, a fifth of
+// them in a caustic, R = 0.2, box):
+//   d, batches of 1.5M queries on maps of 65,536 photons, queries a photon:
+//     k = 8: 0.2 1.34, 0.4 0.98, 0.8 0.74;  k = 32: 0.2 1.20, 0.4 0.82;
+//     k = 64: 0.2 1.41, 0.4 0.96, 0.8 0.68;  k = 128: 0.4 1.41, 0.8 0.95, 1.6 0.72
+//   t, single maps, queries in thousands:
+//     300,001 photons: k = 32: 262 1.15, 400 0.98, 600 0.78;  k = 100: 262 1.11, 400 0.89
+//     1M: k = 1: 900 1.32, 1,300 1.12;  k = 8: 400 1.15, 600 0.96;  k = 32: 400 1.04,
+//         600 0.88;  k = 128: 600 1.22, 900 0.96, 1,300 0.78
+//     4M: k = 32: 900 1.18, 1,300 1.02, 2,000 0.74;  k = 128: 2,000 1.13, 3,000 0.88
+// Photons spread through a volume need more (k = 100: 1M photons, 1.3M queries
+// 1.28), which nothing on the host shows.  Neighbour lists: a warp sorts a group's
+// rows one after another, and where a query finds nearly every photon that is most
+// of the work (k = 100: 128 photons 1.75, 400 1.28, 1,500 and k = 128 1.01).
+double shared_gain(uint32_t n, uint32_t nq, uint32_t k, bool lists) {
+    if (lists && n < 16u * k + 500u) return -(double)nq;
+    const double part = k / 128.0, d = 0.18 + 0.7 / std::sqrt((double)k) + 0.45 * part * part;
+    return std::max(-(double)nq, (double)nq - d * n);   // what is lost is at most the whole
 }
+double shared_tail(uint32_t n, uint32_t k) {
+    return (2e5 + 4.0 * k * k) * std::min(1.0, n / 2.5e5) + 5.5e5 / k * std::min(1.0, n / 2e4);
+}
+bool shared_walk(uint64_t nq, double gain, double tail) { return nq >= 262144u && gain >= tail; }
 
 // k_knn_shared for the launch's queries (a: the wide search's arguments).
 template <bool kBatch>
@@ -1707,7 +1721,7 @@ int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const 
         fx.work_counter = work_counter + 2;
         fx.rounds_per_chunk = 1;
         fx.qsorted = nullptr;
-        if (order && shared_walk(m.n, nq)) {
+        if (order && shared_walk(nq, shared_gain(m.n, nq, p.k, out.nbr != nullptr), shared_tail(m.n, p.k))) {
             launch_shared<false>(a, p.k, nq, t.shared_shapes, st);
         } else {
             const uint32_t grid = grid_for(k_knn_group<32, false, false, true>, threads, smem, nq, t.warps_per_block, a.rounds_per_chunk);
@@ -1778,7 +1792,7 @@ static int launch_batch(const MapView& m, const BatchQuery* bq, const BatchGeom*
     fx.nq_dev = work_counter + 1;
     fx.work_counter = work_counter + 2;
     fx.rounds_per_chunk = 1;
-    if (kW && shared_walk(m.n, nq)) {
+    if (kW && t.qsorted) {   // laid out for the shared walk
         a.qsorted = t.qsorted;
         launch_shared<true>(a, kmax, nq, t.shared_shapes, st);
     } else {

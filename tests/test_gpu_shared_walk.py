@@ -49,15 +49,16 @@ CASES = [
 ]
 
 
+@pytest.mark.parametrize("nbr", [False, True])   # with lists, maps of few photons are searched one by one
 @pytest.mark.parametrize("n,nq,k,r,filt,caustic,cluster,leaf", CASES)
-def test_shared_walk_is_the_single_search(cuda, n, nq, k, r, filt, caustic, cluster, leaf):
+def test_shared_walk_is_the_single_search(cuda, n, nq, k, r, filt, caustic, cluster, leaf, nbr):
     ph = gen.photons(n, seed=n + k, caustic_frac=caustic)
     q = gen.queries(nq, seed=nq, cluster_frac=cluster)
     q.pos[5 % nq, 0] = np.nan   # a query without a position in the middle of a group
     pm = PhotonMap(n, global_q_radius_max=r)
     pm.set_tuning(leaf_size=leaf)
     pm.build(to_dev(ph.pos, cuda), to_dev(ph.pow, cuda))
-    out = both(pm, to_dev(q.pos, cuda), to_dev(q.nrm, cuda), k=k, r_max=r, filter=filt, min_found=3)
+    out = both(pm, to_dev(q.pos, cuda), to_dev(q.nrm, cuda), nbr, k=k, r_max=r, filter=filt, min_found=3)
     assert int(out["count"].max()) > 0
     assert pm.info().device_errors == L.PM_DEVERR_QNONFINITE
 

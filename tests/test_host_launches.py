@@ -106,7 +106,7 @@ def test_shared_memory_limit_is_never_lowered(engine, call, kernel):
 
 @pytest.mark.parametrize("lists", [False, True])
 def test_shared_walk_asks_for_its_block_size_once(engine, lists):
-    n, nq = 1000, 262144
+    n, nq = 3000, 262144
     h = engine.map(n, nq)
     assert engine.build(h, n) == L.PM_OK
     asked = []
@@ -146,7 +146,7 @@ def test_small_sorts_without_room_for_a_cluster(engine, setting, value, n):
 def test_batch_lays_records_out_for_the_shared_walk_only(engine, nq, shared):
     b = C.c_void_p()
     assert engine.lib.pm_batch_create(C.byref(b)) == L.PM_OK
-    photons, queries = (C.c_uint32 * 3)(0, 400, 1000), (C.c_uint32 * 3)(0, 7, nq)
+    photons, queries = (C.c_uint32 * 3)(0, 400, 5000), (C.c_uint32 * 3)(0, 7, nq)
     descs = (L.QueryDesc * 2)(desc(), desc())
     assert engine.lib.pm_batch_build(b, 16, 32, photons, 2, L.PM_PHOTONS_PACKED, None) == L.PM_OK
     engine.log()
@@ -195,3 +195,39 @@ def test_first_adjoint_takes_no_storage_for_photon_records(engine):
     assert len(sizes) == 6 and max(sizes) <= 4 * (n + 1)
     assert launched(log, "k_bwd_prep")
     engine.lib.pm_destroy(h)
+
+
+@pytest.mark.parametrize("n,nq,k,lists,shared", [
+    (1048576, 2073600, 100, False, True), (4194304, 8388608, 64, False, True), (1048576, 1048576, 64, True, True),
+    (250007, 400009, 100, True, True), (3000, 262144, 100, False, True), (3000, 262143, 100, False, False),
+    # sets that were faster one by one: few queries a photon for their k, nearly every photon in every list
+    (1048576, 655360, 128, False, False), (4000000, 1280000, 100, False, False), (600000, 495742, 128, False, False),
+    (65536, 262144, 1, False, False), (1048576, 655360, 1, False, False), (4000000, 2560000, 1, False, False),
+    (100, 524288, 100, True, False), (100, 524288, 50, True, False), (100, 524288, 100, False, True),
+])
+def test_which_queries_share_walks(engine, n, nq, k, lists, shared):
+    h = engine.map(n, nq)
+    assert engine.build(h, n) == L.PM_OK
+    engine.log()
+    assert engine.query(h, nq, lists=lists, k=k) == L.PM_OK
+    assert bool(launched(engine.log(), "k_knn_shared")) == shared
+    engine.lib.pm_destroy(h)
+
+
+@pytest.mark.parametrize("maps,shared", [
+    # (photons, queries, k) of each map: dense, sparse, and both; tiny maps count neither way
+    ([(50000, 200000, 64)] * 3, True), ([(300000, 30000, 64)] * 20, False), ([(300000, 400000, 64), (300000, 30000, 64)], True),
+    ([(300000, 300000, 64)] + [(300000, 60000, 64)] * 10, False), ([(300, 480, 8)] * 3000, False),
+    ([(300, 480, 8)] * 1000 + [(50000, 200000, 64)] * 2, True),
+])
+def test_which_batches_share_walks(engine, maps, shared):
+    b = C.c_void_p()
+    assert engine.lib.pm_batch_create(C.byref(b)) == L.PM_OK
+    off = lambda i: (C.c_uint32 * (len(maps) + 1))(*[sum(m[i] for m in maps[:j]) for j in range(len(maps) + 1)])
+    photons, queries = off(0), off(1)
+    descs = (L.QueryDesc * len(maps))(*[desc(k=m[2]) for m in maps])
+    assert engine.lib.pm_batch_build(b, 16, 32, photons, len(maps), L.PM_PHOTONS_PACKED, None) == L.PM_OK
+    engine.log()
+    assert engine.lib.pm_batch_query(b, descs, 16, 32, queries, 48, None, None, None, None) == L.PM_OK
+    assert bool(launched(engine.log(), "k_knn_shared<true")) == shared
+    assert engine.lib.pm_batch_destroy(b) == L.PM_OK
