@@ -413,10 +413,9 @@ def run_ours(args, cfg, light: bool = False) -> dict | None:
     build_median_ms = rank_max([float(np.median(build_alone))], dev)[0]
 
     kern_ms = float(np.mean(kernels))
+    kernel = pm.query_kernel()
     nodes = info.num_nodes
     alg_bytes = 48 * Q + 32 * N + 64 * (nodes + 1)
-    # sorted sets this large share walks (pm_query.cu, shared_walk)
-    kernel = "k_knn_group" if args.unsorted or Q < 262144 or Q * Q < 409600 * N else "k_knn_shared"
     peak, peak_kind = measured_peaks()
     achieved = alg_bytes / (kern_ms / 1000.0) / 1e9
     build_ms = float(np.mean(builds))

@@ -73,7 +73,7 @@ enum { PM_ORDER_SORTED = 0, PM_ORDER_AS_GIVEN = 1 };
 #define PM_DEVERR_STACK 0x1u     /* traversal stack overflow (query result invalid) */
 #define PM_DEVERR_NONFINITE 0x2u /* non-finite photon position at build */
 #define PM_DEVERR_QNONFINITE 0x4u/* non-finite query position */
-#define PM_DEVERR_WAIT 0x8u      /* a bounded inter-block wait gave up (that call's results are invalid) */
+#define PM_DEVERR_WAIT 0x8u      /* a bounded inter-block wait gave up (kept in the interface; no kernel waits so now) */
 
 typedef struct pm_map pm_map;
 
@@ -121,12 +121,16 @@ PM_API pm_status pm_set_allocator(pm_map* map, pm_alloc_fn alloc, pm_free_fn fre
 /* k-buffer layouts of the query kernel. */
 enum { PM_KBUF_HEAP = 0,   /* one lane per query, max-heap in shared memory */
        PM_KBUF_GROUP = 1,  /* a group of lanes per query, candidate buffer + exact selection */
-       PM_KBUF_WIDE = 2    /* one query per warp over the 32-wide tree, candidate buffer + exact selection */ };
+       PM_KBUF_WIDE = 2    /* over the 32-wide tree: one query per warp, candidate buffer + exact selection;
+                              dense sorted sets share walks, eight queries per warp */ };
 
 /* Tuning knobs (chosen by the autotuner): photons per leaf (1..64), warps per
  * query block (1..8), rounds in the smallest work chunk (1..4096; warps take
- * chunks by guided self-scheduling: long chunks first, this size last), queries per warp
- * (1, 2, 4, 8; group layout) and the k-buffer layout (PM_KBUF_*). */
+ * chunks by guided self-scheduling: long chunks first, this size last; a launch
+ * too small to give every warp one takes shorter chunks), queries per warp
+ * (1, 2, 4, 8; group layout) and the k-buffer layout (PM_KBUF_*).  Shared walks
+ * (PM_KBUF_WIDE) choose their warps per block themselves, and take a quarter of the
+ * rounds, eight queries each. */
 PM_API pm_status pm_set_tuning(pm_map* map, uint32_t leaf_size, int warps_per_block, int rounds_per_chunk,
                                int queries_per_warp, int kbuf_layout);
 
@@ -407,6 +411,11 @@ typedef struct pm_timings {
 } pm_timings;
 PM_API pm_status pm_set_profiling(pm_map* map, int enable);
 PM_API pm_status pm_last_timings(pm_map* map, pm_timings* out);
+
+/* Name of the search kernel that the last kNN search of this handle launched
+ * ("k_knn_shared" where sorted queries shared walks, "k_knn_group", "k_knn_tree"),
+ * "" before the first. */
+PM_API const char* pm_query_kernel(const pm_map* map);
 
 /* Traversal counters of the last pm_query with a binary layout (PM_KBUF_HEAP or
  * PM_KBUF_GROUP; the 32-wide layout keeps no counters), collected

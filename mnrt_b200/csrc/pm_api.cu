@@ -53,6 +53,7 @@ struct pm_map {
     DevBuf qkeys0, qkeys1, qvals0, qvals1, qscratch, counter, fixq, qsorted;
     DevBuf stats;           // query counters (profiling level 2)
     uint32_t shared_shapes[kSharedShapes] = {};   // QueryTuning::shared_shapes
+    const char* query_kernel = "";
     // backward (pm_query_backward): pair sort, per-query records, segments,
     // FP64 running sums, and the forward outputs when the kNN is recomputed
     DevBuf bvals, bvals1, bkeys0, bkeys1, bscratch, blong, qrec, seg_start, seg_end, acc;
@@ -281,6 +282,7 @@ WideBuffers wide_of(pm_map* m) {
 QueryTuning tuning_of(pm_map* m) {
     QueryTuning t;
     t.shared_shapes = m->shared_shapes;
+    t.kernel = &m->query_kernel;
     t.layout = m->kbuf_layout;
     t.queries_per_warp = m->queries_per_warp;
     t.warps_per_block = m->warps_per_block;
@@ -1055,6 +1057,8 @@ pm_status pm_set_profiling(pm_map* m, int enable) {
     m->profile_level = enable;
     return PM_OK;
 }
+
+const char* pm_query_kernel(const pm_map* m) { return m ? m->query_kernel : ""; }
 
 pm_status pm_query_stats(pm_map* m, uint64_t* out, uint32_t count) {
     if (!m || !out) return fail(m, PM_ERR_INVALID, "stats output is NULL");

@@ -180,6 +180,7 @@ struct QueryTuning {
     int warps_per_block;
     int rounds_per_chunk;
     unsigned long long* stats;   // 8 traversal counters (group layout), nullptr = off
+    const char** kernel;         // set to the search kernel's name
     uint32_t* shared_shapes;     // the handle's launch shapes of the shared walk (kSharedShapes words, 0: not asked yet)
     const float4* qsorted = nullptr;   // query records in sorted order (pos.xyz | caller index, normal), or nullptr
                                        // (a batch: set where it shares walks)

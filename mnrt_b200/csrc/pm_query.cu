@@ -1695,6 +1695,7 @@ int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const 
     if (!nq) return 0;
     KnnArgs a = make_args(m, p, qpos, qnrm, order, nq, out);
     a.work_counter = work_counter;
+    *t.kernel = "k_knn_group";
     a.stats = t.stats;
     if (t.stats) cudaMemsetAsync(t.stats, 0, kStatCount * sizeof(unsigned long long), st);
     a.rounds_per_chunk = (uint32_t)t.rounds_per_chunk;
@@ -1704,6 +1705,7 @@ int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const 
         const int smem = query_smem_bytes_per_warp(p.k) * t.warps_per_block;
         const uint32_t grid = grid_for(k_knn_tree, threads, smem, (nq + 31u) / 32u, t.warps_per_block, a.rounds_per_chunk);
         k_knn_tree<<<grid, threads, smem, st>>>(a);
+        *t.kernel = "k_knn_tree";
         return 1;
     }
     if (t.layout == 2) {   // over the 32-wide tree
@@ -1723,6 +1725,7 @@ int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const 
         fx.qsorted = nullptr;
         if (order && shared_walk(nq, shared_gain(m.n, nq, p.k, out.nbr != nullptr), shared_tail(m.n, p.k))) {
             launch_shared<false>(a, p.k, nq, t.shared_shapes, st);
+            *t.kernel = "k_knn_shared";
         } else {
             const uint32_t grid = grid_for(k_knn_group<32, false, false, true>, threads, smem, nq, t.warps_per_block, a.rounds_per_chunk);
             k_knn_group<32, false, false, true><<<grid, threads, smem, st>>>(a);
@@ -1787,6 +1790,7 @@ static int launch_batch(const MapView& m, const BatchQuery* bq, const BatchGeom*
     const int threads = 32 * t.warps_per_block;
     const int smem = (int)a.smem_per_warp * t.warps_per_block;
     cudaMemsetAsync(work_counter, 0, 3 * sizeof(uint32_t), st);
+    *t.kernel = kW && t.qsorted ? "k_knn_shared" : "k_knn_group";
     KnnArgs fx = a;   // queries whose estimate needs FP64 distances, or that the shared walk left
     fx.fix_in = fix_list;
     fx.nq_dev = work_counter + 1;

@@ -206,6 +206,10 @@ class PhotonMap:
         L.check(self._lib.pm_query_stats(self._h, out.ctypes.data, 8), self._h)
         return dict(zip(self.STAT_NAMES, (int(x) for x in out)))
 
+    def query_kernel(self) -> str:
+        """Name of the search kernel of this map's last kNN search ("" before the first)."""
+        return self._lib.pm_query_kernel(self._h).decode()
+
     def last_timings(self) -> L.Timings:
         t = L.Timings()
         L.check(self._lib.pm_last_timings(self._h, C.byref(t)), self._h)

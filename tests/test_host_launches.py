@@ -211,6 +211,7 @@ def test_which_queries_share_walks(engine, n, nq, k, lists, shared):
     engine.log()
     assert engine.query(h, nq, lists=lists, k=k) == L.PM_OK
     assert bool(launched(engine.log(), "k_knn_shared")) == shared
+    assert engine.lib.pm_query_kernel(h) == (b"k_knn_shared" if shared else b"k_knn_group")
     engine.lib.pm_destroy(h)
 
 
