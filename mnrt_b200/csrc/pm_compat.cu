@@ -29,13 +29,16 @@
 // farthest possible distances fall into one histogram bin is counted as a
 // whole (the bin is a monotone function of d^2, and both bounds are rounded as
 // d^2 is), so a dense blob far from the centre costs a step per 32 leaves and
-// not one per photon.  The root-to-leaf path of a query is a lane's: a warp
-// takes several queries, descends for all of them at once and then refines and
-// gathers one after the other.  With a thread per query and per slot instead
-// the kernels ran at the pace of the slots beside the blob: 300,001 photons (20 %
-// in a caustic of sigma 0.01), 307,200 queries, k = 50, R = 0.1, build included:
-// 54.9 -> 3.37 ms; 1,500 photons and 4,000 radii: 350 -> 140 us.  Latency bounds
-// what is left (dependent node loads; a quarter of the warps' slots is taken).
+// not one per photon.  The root-to-leaf path of a query is a thread's.  With a
+// thread per query and per slot throughout the kernels ran at the pace of the
+// slots beside the blob: 300,001 photons (20 % in a caustic of sigma 0.01),
+// 307,200 queries, k = 50, R = 0.1, build included: 54.9 -> 2.9 ms; 1,500 photons
+// and 4,000 radii: 350 -> 79 us.  Latency bounds what is left (dependent node
+// loads; a quarter of the warps' slots is taken).
+//
+// Ranges of no more than two leaves are the exception: a warp has 30 lanes too
+// many for them, and where there are many queries a thread each answers more
+// (k_compat_start).
 #include "pm_internal.h"
 
 namespace pm {
@@ -154,6 +157,18 @@ __device__ __forceinline__ bool warp_range(const MapView& m, float qx, float qy,
     return true;
 }
 
+// The histogram's bin of a squared distance in [lo, lo + delta]: monotone in d^2.
+__device__ __forceinline__ uint32_t hist_bin(float d2, float lo, float delta) {
+    const float fi = __fdiv_rn(__fmul_rn(fmaxf(__fsub_rn(__fsqrt_rn(d2), lo), 0.0f), (float)kHist), delta);
+    return min((uint32_t)fi, kHist - 1u);
+}
+// Narrows [r_min, r_max] to bin mb.
+__device__ __forceinline__ void narrow(float& r_min, float& r_max, float delta, uint32_t mb) {
+    const float lo = r_min, inv = 1.0f / (float)kHist;
+    r_min = __fadd_rn(lo, __fmul_rn(__fmul_rn((float)mb, delta), inv));
+    r_max = __fadd_rn(lo, __fmul_rn(__fmul_rn((float)(mb + 1), delta), inv));
+}
+
 // Zhou et al. 2008 histogram refinement of a query radius, by a warp.
 __device__ float refine_radius(const MapView& m, float qx, float qy, float qz, float radius_max, uint32_t k,
                                uint32_t iters, CompatSmem& s, uint32_t lane, bool& ok) {
@@ -163,26 +178,21 @@ __device__ float refine_radius(const MapView& m, float qx, float qy, float qz, f
     // tested one by one.
     const bool one_by_one = m.hdr->nonfinite != 0;
     for (uint32_t it = 0; it < iters; ++it) {
-        const float r = r_max, lo = r_min;
-        const float delta = __fsub_rn(r_max, r_min);
+        const float lo = r_min, delta = __fsub_rn(r_max, r_min);
         if (!(delta > 0.0f)) break;
         s.hist[lane] = 0;
         __syncwarp();
-        auto bin = [&](float d2) {   // monotone in d^2
-            const float fi = __fdiv_rn(__fmul_rn(fmaxf(__fsub_rn(__fsqrt_rn(d2), lo), 0.0f), (float)kHist), delta);
-            return min((uint32_t)fi, kHist - 1u);
-        };
-        const float r2 = __fmul_rn(r, r);
+        const float r2 = __fmul_rn(r_max, r_max);
         ok = warp_range(m, qx, qy, qz, r2, s, lane,
                         [&](float lb, float ub, uint32_t cnt) {
                             if (one_by_one || !(ub < r2)) return false;
-                            const uint32_t b = bin(lb);
-                            if (b != bin(ub)) return false;
+                            const uint32_t b = hist_bin(lb, lo, delta);
+                            if (b != hist_bin(ub, lo, delta)) return false;
                             atomicAdd(&s.hist[b], cnt);
                             return true;
                         },
                         [&](bool in, uint32_t, float d2) {
-                            if (in) atomicAdd(&s.hist[bin(d2)], 1u);
+                            if (in) atomicAdd(&s.hist[hist_bin(d2, lo, delta)], 1u);
                         }) && ok;
         uint32_t sum = min(s.hist[lane], 0xfffeu);   // the reference's counters saturate
 #pragma unroll
@@ -191,10 +201,7 @@ __device__ float refine_radius(const MapView& m, float qx, float qy, float qz, f
             if (lane >= (uint32_t)o) sum += y;
         }
         const uint32_t reach = __ballot_sync(kFull, sum >= k);
-        const uint32_t mb = reach ? (uint32_t)__ffs(reach) - 1u : kHist - 1u;
-        const float inv = 1.0f / (float)kHist;
-        r_min = __fadd_rn(lo, __fmul_rn(__fmul_rn((float)mb, delta), inv));
-        r_max = __fadd_rn(lo, __fmul_rn(__fmul_rn((float)(mb + 1), delta), inv));
+        narrow(r_min, r_max, delta, reach ? (uint32_t)__ffs(reach) - 1u : kHist - 1u);
         __syncwarp();
     }
     return r_max;
@@ -233,9 +240,12 @@ __global__ void __launch_bounds__(32 * kCompatWarps) k_compat_nodes(MapView m, u
     }
 }
 
-// The radius a query starts from (one lane's descent).
-__device__ float path_radius(const Node* nodes, const float* est, float qx, float qy, float qz, float rmax) {
+// The radius a query starts from (a thread's descent), and the radius of the box
+// the descent ends in.
+__device__ float path_radius(const Node* nodes, const float* est, float qx, float qy, float qz, float rmax,
+                             float& leaf_rad) {
     float e = rmax;
+    leaf_rad = 0.0f;
     uint32_t sid = 0;
     float lo[3], hi[3];
     uint32_t ref, cnt;
@@ -246,6 +256,7 @@ __device__ float path_radius(const Node* nodes, const float* est, float qx, floa
         extent_of(lo, hi, c, rad);
         const float len = __fsqrt_rn(d2_rn(qx, qy, qz, c[0], c[1], c[2]));
         e = fminf(e, __fadd_rn(len, est[sid]));
+        leaf_rad = rad;
         if (cnt > 0) break;
         float l1[3], h1[3];
         uint32_t r1, c1;
@@ -264,7 +275,7 @@ __device__ float path_radius(const Node* nodes, const float* est, float qx, floa
     return e;
 }
 
-struct CompatArgs {
+struct CompatArgs {   // out_rad and what goes with it, or out_radius alone
     MapView m;
     const float* est;
     const float4* qpos;
@@ -280,6 +291,196 @@ struct CompatArgs {
     uint32_t* out_count;
 };
 
+// The scaled integer sums of one estimate: their order does not matter.
+struct CompatFlux {
+    double qx, qy, qz, r2, kc;
+    float scale;   // 2^40 / max flux: a range may hold far more than 128 photons
+    float4 qn;
+    long long c0 = 0, c1 = 0, c2 = 0;
+    __device__ __forceinline__ void begin(const CompatArgs& a, float x, float y, float z, const float4& n, float r2u) {
+        qx = x; qy = y; qz = z; r2 = r2u; kc = a.cone_k; qn = n;
+        scale = __fmul_rn(a.m.hdr->fix_scale, 1.220703125e-4f);
+    }
+    __device__ __forceinline__ void add(const CompatArgs& a, uint32_t t) {
+        const float4 w = __ldg(a.m.pow + t);
+        if (!front_rn(qn.x, qn.y, qn.z, __float_as_uint(w.w))) return;
+        const float4 p = __ldg(a.m.pos + t);
+        const double dx = (double)p.x - qx, dy = (double)p.y - qy, dz = (double)p.z - qz;
+        const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+        double wt = 1.0;
+        if (a.filter == 1) wt = 1.0 - __dsqrt_rn(d2) / (kc * __dsqrt_rn(r2));
+        else if (a.filter == 2) wt = 1.0 - d2 / r2;
+        c0 += __double2ll_rn(wt * (double)w.x * (double)scale);
+        c1 += __double2ll_rn(wt * (double)w.y * (double)scale);
+        c2 += __double2ll_rn(wt * (double)w.z * (double)scale);
+    }
+    __device__ __forceinline__ void result(const CompatArgs& a, float4& rad) const {
+        if (!(scale > 0.0f)) return;
+        const double pi = 3.14159265358979323846;
+        double norm = 1.0 / (pi * r2);
+        if (a.filter == 1) norm = 1.0 / ((1.0 - 2.0 / (3.0 * kc)) * pi * r2);
+        else if (a.filter == 2) norm = 2.0 / (pi * r2);
+        const double f = norm / (double)scale;
+        rad.x = __double2float_rn((double)c0 * f);
+        rad.y = __double2float_rn((double)c1 * f);
+        rad.z = __double2float_rn((double)c2 * f);
+    }
+};
+
+__device__ __forceinline__ void compat_store(const CompatArgs& a, uint32_t q, float r, const float4& rad, float r2u,
+                                             uint32_t count) {
+    if (a.out_radius) a.out_radius[q] = r;
+    if (!a.out_rad) return;
+    a.out_rad[q] = rad;
+    if (a.out_r2) a.out_r2[q] = r2u;
+    if (a.out_count) a.out_count[q] = count;
+}
+
+// A query that k_compat_start leaves to its warp: its start radius r > 0 waits where
+// its result will be.
+__device__ __forceinline__ void compat_defer(const CompatArgs& a, uint32_t q, float r) {
+    if (a.out_rad) a.out_rad[q] = make_float4(r, 0.0f, 0.0f, -1.0f);
+    else a.out_radius[q] = -r;
+}
+__device__ __forceinline__ bool compat_deferred(const CompatArgs& a, uint32_t q, float& r) {
+    if (a.out_rad) {
+        const float4 v = a.out_rad[q];
+        r = v.x;
+        return v.w < 0.0f;
+    }
+    r = -a.out_radius[q];
+    return r > 0.0f;
+}
+
+// Leaves a thread lists for its own range, and their photons at most (a bit each).
+constexpr uint32_t kOwnLeaves = 2, kOwnPhotons = 64, kOwnStack = 24, kOwnSteps = 64;
+constexpr int kOwnThreads = 128;
+// Queries from which threads answer first: below, a launch's warps are not all taken,
+// and a warp answers one query sooner (maps of no more than a leaf: 20,000 queries,
+// 64 photons, R = 0.1, a warp each 23 us, a thread each 11).
+constexpr uint32_t kOwnMin = 65536, kOwnMinFew = 16384;
+
+// A query's position and start radius; false where it is answered (a position that
+// is not finite, a radius of zero).
+__device__ __forceinline__ bool compat_begin(const CompatArgs& a, uint32_t q, float4& qp, float& r0, float& leaf_rad) {
+    qp = a.qpos[q];
+    r0 = a.rmax;
+    const bool fin = isfinite(qp.x) && isfinite(qp.y) && isfinite(qp.z);
+    if (fin) r0 = path_radius(a.m.nodes, a.est, qp.x, qp.y, qp.z, a.rmax, leaf_rad);
+    else atomicOr(&a.m.hdr->errors, kErrQueryNonFinite);
+    if (fin && r0 > 0.0f) return true;
+    compat_store(a, q, r0, make_float4(0.0f, 0.0f, 0.0f, 0.0f), __fmul_rn(r0, r0), 0u);
+    return false;
+}
+
+// Thread per query: the start radius, and the whole answer where the range is a
+// leaf or two (start radius a quarter of the query's own leaf's, or a map of no more
+// than a leaf): the leaves are listed by one descent, as every later radius is
+// smaller, and their photons tested in place.  The other queries are left to
+// k_compat_query.  1M queries, a warp for each / this, us: 64 photons, R = 0.1 512 / 70;
+// 1,500 photons, R = 0.02 672 / 180; 20,000 photons, R = 0.003 795 / 291.  Ranges of
+// more photons are slower by a thread's chain of tests (500 queries, 100,000 photons,
+// R = 0.02, up to 160 photons: 17 / 130 us), so few queries take a warp each.
+__global__ void __launch_bounds__(kOwnThreads) k_compat_start(CompatArgs a) {
+    __shared__ uint32_t s_hist[kHist / 4][kOwnThreads];   // byte counters, a column per thread
+    const uint64_t q64 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q64 >= a.nq) return;
+    const uint32_t q = (uint32_t)q64, me = threadIdx.x;
+    float4 qp;
+    float r0, leaf_rad;
+    if (!compat_begin(a, q, qp, r0, leaf_rad)) return;
+    uint32_t ref[kOwnLeaves], cnt[kOwnLeaves], leaves = 0, photons = 0;
+    bool own = a.m.n <= kLeafMax || 4.0f * r0 <= leaf_rad;
+    if (a.m.n <= kLeafMax) {
+        ref[0] = 0;
+        cnt[0] = a.m.n;
+        leaves = 1;
+    } else if (own) {
+        const float r2 = __fmul_rn(r0, r0);
+        uint32_t stack[kOwnStack], sp = 1, steps = 0;
+        stack[0] = 0u;
+        while (sp > 0 && own) {
+            float lo[3], hi[3];
+            uint32_t kid, c;
+            slot_of(a.m.nodes, stack[--sp], lo, hi, kid, c);
+            if (kid != kInvalid && box_lb(qp.x, qp.y, qp.z, lo, hi) < r2) {
+                if (c > 0) {
+                    photons += c;
+                    own = leaves < kOwnLeaves && photons <= kOwnPhotons;
+                    if (own) { ref[leaves] = kid; cnt[leaves] = c; ++leaves; }
+                } else {
+                    own = sp + 2 <= kOwnStack;
+                    if (own) { stack[sp++] = kid << 1 | 1u; stack[sp++] = kid << 1; }
+                }
+            }
+            own = own && ++steps < kOwnSteps;
+        }
+    }
+    if (!own) {
+        compat_defer(a, q, r0);
+        return;
+    }
+    auto each = [&](float r2, auto&& f) {   // the listed photons with d^2 < r2, four loads in flight
+        uint32_t first = 0;
+#pragma unroll 1
+        for (uint32_t l = 0; l < leaves; ++l) {
+#pragma unroll 1
+            for (uint32_t j = 0; j < cnt[l]; j += 4) {
+                float4 p[4];
+#pragma unroll
+                for (uint32_t u = 0; u < 4; ++u) p[u] = __ldg(a.m.pos + ref[l] + min(j + u, cnt[l] - 1u));
+#pragma unroll
+                for (uint32_t u = 0; u < 4; ++u) {
+                    const float d2 = d2_rn(qp.x, qp.y, qp.z, p[u].x, p[u].y, p[u].z);
+                    if (j + u < cnt[l] && d2 < r2) f(first + j + u, d2);
+                }
+            }
+            first += cnt[l];
+        }
+    };
+    float r_min = 0.0f, r_max = r0;
+    for (uint32_t it = 0; it < a.iters; ++it) {
+        const float lo = r_min, delta = __fsub_rn(r_max, r_min);
+        if (!(delta > 0.0f)) break;
+        for (uint32_t b = 0; b < kHist / 4; ++b) s_hist[b][me] = 0;
+        each(__fmul_rn(r_max, r_max), [&](uint32_t, float d2) {
+            const uint32_t b = hist_bin(d2, lo, delta);
+            s_hist[b >> 2][me] += 1u << ((b & 3u) * 8u);
+        });
+        uint32_t mb = 0, sum = 0;
+        for (; mb < kHist - 1u; ++mb) {
+            sum += (s_hist[mb >> 2][me] >> ((mb & 3u) * 8u)) & 255u;
+            if (sum >= a.k) break;
+        }
+        narrow(r_min, r_max, delta, mb);
+    }
+    if (!a.out_rad) {
+        a.out_radius[q] = r_max;
+        return;
+    }
+    const float r2 = __fmul_rn(r_max, r_max);
+    uint64_t found = 0;   // a bit per listed photon
+    float maxd2 = 0.0f;
+    each(r2, [&](uint32_t i, float d2) { found |= 1ull << i; maxd2 = fmaxf(maxd2, d2); });
+    const uint32_t count = (uint32_t)__popcll(found);
+    const float r2u = count >= a.k ? maxd2 : r2;
+    float4 rad = make_float4(0.0f, 0.0f, 0.0f, (float)count);
+    if (count > 0 && count >= a.min_found && r2u > 0.0f) {
+        CompatFlux flux;
+        flux.begin(a, qp.x, qp.y, qp.z, a.qnrm[q], r2u);
+#pragma unroll 1
+        for (; found; found &= found - 1) {
+            const uint32_t i = (uint32_t)__ffsll((long long)found) - 1u;
+            flux.add(a, i < cnt[0] ? ref[0] + i : ref[1] + (i - cnt[0]));
+        }
+        flux.result(a, rad);
+    }
+    compat_store(a, q, r_max, rad, r2u, count);
+}
+
+// A warp per query, per_warp queries after one another: those that k_compat_start
+// left (kStarted), or all of them, each lane descending for one first.
+template <bool kStarted>
 __global__ void __launch_bounds__(32 * kCompatWarps, 4) k_compat_query(CompatArgs a) {
     __shared__ CompatSmem s_warp[kCompatWarps];
     const uint32_t lane = lane_id(), lt = (1u << lane) - 1u;
@@ -288,91 +489,64 @@ __global__ void __launch_bounds__(32 * kCompatWarps, 4) k_compat_query(CompatArg
     if (q0 >= a.nq) return;
     const uint32_t nw = (uint32_t)min((uint64_t)a.per_warp, (uint64_t)a.nq - q0);
     float4 qp = make_float4(0.f, 0.f, 0.f, 0.f);
-    float e0 = a.rmax;
-    bool fin = false;
-    if (lane < nw) {   // a query per lane: its start radius
-        qp = a.qpos[q0 + lane];
-        fin = isfinite(qp.x) && isfinite(qp.y) && isfinite(qp.z);
-        if (fin) e0 = path_radius(a.m.nodes, a.est, qp.x, qp.y, qp.z, a.rmax);
-        else atomicOr(&a.m.hdr->errors, kErrQueryNonFinite);
+    float e0 = 0.0f;
+    bool mine = false;
+    if (lane < nw) {
+        if constexpr (kStarted) {
+            mine = compat_deferred(a, (uint32_t)q0 + lane, e0);
+            if (mine) qp = a.qpos[q0 + lane];
+        } else {
+            float leaf_rad;
+            mine = compat_begin(a, (uint32_t)q0 + lane, qp, e0, leaf_rad);
+        }
     }
+    uint32_t todo = __ballot_sync(kFull, mine);
     bool ok = true;
-    for (uint32_t i = 0; i < nw; ++i) {
-        const uint32_t q = (uint32_t)q0 + i;
+    for (; todo; todo &= todo - 1u) {
+        const int i = __ffs(todo) - 1;
+        const uint32_t q = (uint32_t)q0 + (uint32_t)i;
         const float qx = __shfl_sync(kFull, qp.x, i), qy = __shfl_sync(kFull, qp.y, i), qz = __shfl_sync(kFull, qp.z, i);
-        const bool finite = __shfl_sync(kFull, fin ? 1 : 0, i);
-        float r = __shfl_sync(kFull, e0, i);
-        if (finite) r = refine_radius(a.m, qx, qy, qz, r, a.k, a.iters, s, lane, ok);
-        if (a.out_radius && lane == 0) a.out_radius[q] = r;
-        if (!a.out_rad) continue;
+        const float r = refine_radius(a.m, qx, qy, qz, __shfl_sync(kFull, e0, i), a.k, a.iters, s, lane, ok);
+        if (!a.out_rad) {
+            if (lane == 0) a.out_radius[q] = r;
+            continue;
+        }
         const float r2 = __fmul_rn(r, r);
         uint32_t count = 0;   // photons in range; the first kCompatKeep are kept
         float maxd2 = 0.0f;
         auto none = [](float, float, uint32_t) { return false; };
-        if (finite) {
-            ok = warp_range(a.m, qx, qy, qz, r2, s, lane, none,
-                            [&](bool in, uint32_t t, float d2) {
-                                const uint32_t bal = __ballot_sync(kFull, in);
-                                const uint32_t at = count + __popc(bal & lt);
-                                if (in) {
-                                    maxd2 = fmaxf(maxd2, d2);
-                                    if (at < kCompatKeep) s.keep[at] = t;
-                                }
-                                count += __popc(bal);
-                            }) && ok;
-            maxd2 = __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(maxd2)));
-        }
+        ok = warp_range(a.m, qx, qy, qz, r2, s, lane, none,
+                        [&](bool in, uint32_t t, float d2) {
+                            const uint32_t bal = __ballot_sync(kFull, in);
+                            const uint32_t at = count + __popc(bal & lt);
+                            if (in) {
+                                maxd2 = fmaxf(maxd2, d2);
+                                if (at < kCompatKeep) s.keep[at] = t;
+                            }
+                            count += __popc(bal);
+                        }) && ok;
+        maxd2 = __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(maxd2)));
         const float r2u = count >= a.k ? maxd2 : r2;
         float4 rad = make_float4(0.0f, 0.0f, 0.0f, (float)count);
-        if (finite && count > 0 && count >= a.min_found && r2u > 0.0f) {
-            const float4 qn = a.qnrm[q];
-            const double r2d = (double)r2u;
-            const double kc = (double)a.cone_k;
-            // 2^40 / max flux: a range may hold far more than 128 photons
-            const float scale = __fmul_rn(a.m.hdr->fix_scale, 1.220703125e-4f);
-            long long c0 = 0, c1 = 0, c2 = 0;
-            auto add = [&](uint32_t t) {
-                const float4 w = __ldg(a.m.pow + t);
-                if (!front_rn(qn.x, qn.y, qn.z, __float_as_uint(w.w))) return;
-                const float4 p = __ldg(a.m.pos + t);
-                const double dx = (double)p.x - (double)qx, dy = (double)p.y - (double)qy, dz = (double)p.z - (double)qz;
-                const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-                double wt = 1.0;
-                if (a.filter == 1) wt = 1.0 - __dsqrt_rn(d2) / (kc * __dsqrt_rn(r2d));
-                else if (a.filter == 2) wt = 1.0 - d2 / r2d;
-                c0 += __double2ll_rn(wt * (double)w.x * (double)scale);
-                c1 += __double2ll_rn(wt * (double)w.y * (double)scale);
-                c2 += __double2ll_rn(wt * (double)w.z * (double)scale);
-            };
+        if (count > 0 && count >= a.min_found && r2u > 0.0f) {
+            CompatFlux flux;
+            flux.begin(a, qx, qy, qz, a.qnrm[q], r2u);
             if (count <= kCompatKeep) {
-                for (uint32_t e = lane; e < count; e += 32) add(s.keep[e]);
+                for (uint32_t e = lane; e < count; e += 32) flux.add(a, s.keep[e]);
             } else {
                 warp_range(a.m, qx, qy, qz, r2, s, lane, none, [&](bool in, uint32_t t, float) {
-                    if (in) add(t);
+                    if (in) flux.add(a, t);
                 });
             }
 #pragma unroll
             for (int o = 16; o; o >>= 1) {
-                c0 += __shfl_xor_sync(kFull, c0, o);
-                c1 += __shfl_xor_sync(kFull, c1, o);
-                c2 += __shfl_xor_sync(kFull, c2, o);
+                flux.c0 += __shfl_xor_sync(kFull, flux.c0, o);
+                flux.c1 += __shfl_xor_sync(kFull, flux.c1, o);
+                flux.c2 += __shfl_xor_sync(kFull, flux.c2, o);
             }
-            if (scale > 0.0f) {
-                const double pi = 3.14159265358979323846;
-                double norm = 1.0 / (pi * r2d);
-                if (a.filter == 1) norm = 1.0 / ((1.0 - 2.0 / (3.0 * kc)) * pi * r2d);
-                else if (a.filter == 2) norm = 2.0 / (pi * r2d);
-                const double f = norm / (double)scale;
-                rad.x = __double2float_rn((double)c0 * f);
-                rad.y = __double2float_rn((double)c1 * f);
-                rad.z = __double2float_rn((double)c2 * f);
-            }
+            flux.result(a, rad);
         }
-        if (lane == 0) {
-            a.out_rad[q] = rad;
-            if (a.out_r2) a.out_r2[q] = r2u;
-            if (a.out_count) a.out_count[q] = count;
-        }
+        if (lane == 0) compat_store(a, q, r, rad, r2u, count);
         __syncwarp();   // keep is reused
     }
     if (!ok && lane == 0) atomicOr(&a.m.hdr->errors, kErrStack);
@@ -405,13 +579,21 @@ int compat_query(const MapView& m, const float* est, const QueryParams& p, uint3
     a.qpos = qpos; a.qnrm = qnrm; a.nq = nq; a.k = p.k; a.iters = iters; a.min_found = p.min_found;
     a.rmax = p.r; a.filter = p.filter; a.cone_k = p.cone_k;
     a.out_radius = out_radius; a.out_rad = out.rad; a.out_r2 = out.r2; a.out_count = out.count;
-    // as many queries per warp as leave about four waves of warps (56 per SM)
-    const uint32_t warps = 4u * 56u * (uint32_t)sm_count();
+    // as many queries per warp as leave about seven waves of the 32 warps that shared
+    // memory lets an SM hold
+    const uint32_t warps = 7u * 32u * (uint32_t)sm_count();
     a.per_warp = 1;
     while (a.per_warp < 32 && nq / (a.per_warp * 2u) >= warps) a.per_warp *= 2u;
     const uint32_t per_block = a.per_warp * kCompatWarps;
-    k_compat_query<<<(nq + per_block - 1) / per_block, 32 * kCompatWarps, 0, st>>>(a);
-    return 1;
+    const uint32_t grid = (nq + per_block - 1) / per_block;
+    if (nq < (m.n <= kLeafMax ? kOwnMinFew : kOwnMin)) {
+        k_compat_query<false><<<grid, 32 * kCompatWarps, 0, st>>>(a);
+        return 1;
+    }
+    k_compat_start<<<(nq + kOwnThreads - 1) / kOwnThreads, kOwnThreads, 0, st>>>(a);
+    if (m.n <= kLeafMax) return 1;   // answered whole
+    k_compat_query<true><<<grid, 32 * kCompatWarps, 0, st>>>(a);
+    return 2;
 }
 
 }  // namespace pm

@@ -8,6 +8,7 @@ import threading
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
+import numpy as np
 import pytest
 
 from mnrt_b200 import _lib as L
@@ -232,3 +233,18 @@ def test_which_batches_share_walks(engine, maps, shared):
     assert engine.lib.pm_batch_query(b, descs, 16, 32, queries, 48, None, None, None, None) == L.PM_OK
     assert bool(launched(engine.log(), "k_knn_shared<true")) == shared
     assert engine.lib.pm_batch_destroy(b) == L.PM_OK
+
+
+@pytest.mark.parametrize("n,nq,kernels", [
+    (64, 16383, ["k_compat_query<false>"]), (64, 16384, ["k_compat_start"]),
+    (65, 65535, ["k_compat_query<false>"]), (65, 65536, ["k_compat_start", "k_compat_query<true>"]),
+])
+def test_many_small_ranges_are_answered_by_threads(engine, n, nq, kernels):
+    """A warp for each of many queries with a photon or two in range took up to 26 times a
+    thread's share of the chip."""
+    h = engine.map(n, nq)
+    assert engine.build(h, n) == L.PM_OK
+    engine.log()
+    assert engine.query(h, nq, mode=L.PM_MODE_ZHOU_COMPAT) == L.PM_OK
+    assert [x.split(" grid")[0].split(" ", 1)[1] for x in engine.log() if " k_compat_" in x][1:] == kernels   # after the nodes
+    engine.lib.pm_destroy(h)
