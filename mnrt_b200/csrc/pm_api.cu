@@ -1552,14 +1552,15 @@ struct TuneCand {
     int wpb, rounds, qpw, layout;
 };
 
+constexpr uint32_t kTuneLeaves[] = {16, 24, 32, 48, 64};
+constexpr int kTuneWarps[] = {2, 4, 8};
+constexpr int kTuneRounds[] = {8, 32};
+
 std::vector<TuneCand> tune_candidates(uint32_t k) {
     std::vector<TuneCand> c;
-    const uint32_t leaves[] = {16, 24, 32, 48, 64};
-    const int wpbs[] = {2, 4, 8};
-    const int rounds[] = {8, 32};
-    for (uint32_t l : leaves)
-        for (int w : wpbs)
-            for (int r : rounds) {
+    for (uint32_t l : kTuneLeaves)
+        for (int w : kTuneWarps)
+            for (int r : kTuneRounds) {
                 c.push_back({l, w, r, 1, PM_KBUF_GROUP});
                 c.push_back({l, w, r, 2, PM_KBUF_GROUP});
                 c.push_back({l, w, r, 1, PM_KBUF_WIDE});
@@ -1605,7 +1606,15 @@ extern "C" pm_status pm_autotune(pm_map* m, const float* d_pos4, const float* d_
     TuneCand best_c{saved_leaf, saved[0], saved[1], saved[2], saved[3]};
     float best_b = 0, best_q = 0;
     const double scale = (double)nq / (double)sample;
-    for (const TuneCand& c : tune_candidates(desc->k)) {
+    // where the sample shares walks the search chooses its own warps per block: one
+    // candidate then stands for all of them, with the setting the map has
+    const bool shares = desc->order == PM_ORDER_SORTED &&
+                        shared_walk(sample, shared_gain(n, sample, desc->k, false), shared_tail(n, desc->k));
+    for (TuneCand c : tune_candidates(desc->k)) {
+        if (shares && c.layout == PM_KBUF_WIDE) {
+            if (c.wpb != kTuneWarps[0]) continue;
+            c.wpb = saved[0];
+        }
         m->leaf_size = c.leaf; m->warps_per_block = c.wpb; m->rounds_per_chunk = c.rounds;
         m->queries_per_warp = c.qpw; m->kbuf_layout = c.layout;
         float tb = 0, tq = 0;
@@ -1659,16 +1668,18 @@ extern "C" pm_status pm_batch_autotune(pm_batch* b, const float* d_pos4, const f
     uint32_t bl = saved_leaf;
     int bw = saved_wpb, br = saved_rounds;
     pm_status s = PM_OK;
-    const uint32_t leaves[] = {16, 24, 32, 48, 64};
-    const int wpbs[] = {2, 4, 8};
-    const int rounds[] = {8, 32};
     const int layouts[] = {PM_KBUF_GROUP, PM_KBUF_WIDE};
     int blay = PM_KBUF_WIDE;
-    for (uint32_t l : leaves)
-        for (int w : wpbs)
-            for (int r : rounds)
+    for (uint32_t l : kTuneLeaves)
+        for (int w : kTuneWarps)
+            for (int r : kTuneRounds)
               for (int lay : layouts) {
-                m->leaf_size = l; m->warps_per_block = w; m->rounds_per_chunk = r;
+                // b->shared is known from the first candidate's queries (a shared walk
+                // chooses its own warps per block: the batch's setting stands for all)
+                const bool own_warps = lay == PM_KBUF_WIDE && b->shared[0];
+                if (own_warps && w != kTuneWarps[0]) continue;
+                const int wpb = own_warps ? saved_wpb : w;
+                m->leaf_size = l; m->warps_per_block = wpb; m->rounds_per_chunk = r;
                 m->queries_per_warp = 1; m->kbuf_layout = lay;
                 float tb = 0, tq = 0;
                 for (int rep = 0; rep < 2 && s == PM_OK; ++rep) {
@@ -1685,7 +1696,7 @@ extern "C" pm_status pm_batch_autotune(pm_batch* b, const float* d_pos4, const f
                 }
                 if (s != PM_OK) break;
                 if (tb + tq < best_score) {
-                    best_score = tb + tq; bl = l; bw = w; br = r; blay = lay; best_b = tb; best_q = tq;
+                    best_score = tb + tq; bl = l; bw = wpb; br = r; blay = lay; best_b = tb; best_q = tq;
                 }
               }
     for (cudaEvent_t& e : ev) cudaEventDestroy(e);

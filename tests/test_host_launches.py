@@ -248,3 +248,31 @@ def test_many_small_ranges_are_answered_by_threads(engine, n, nq, kernels):
     assert engine.query(h, nq, mode=L.PM_MODE_ZHOU_COMPAT) == L.PM_OK
     assert [x.split(" grid")[0].split(" ", 1)[1] for x in engine.log() if " k_compat_" in x][1:] == kernels   # after the nodes
     engine.lib.pm_destroy(h)
+
+
+def test_autotuners_time_a_shared_walk_once_per_leaf_and_rounds(engine):
+    """A shared walk chooses its own warps per block: timing it for each setting would
+    pick among equals by noise, and leave searches one by one with that setting."""
+    n, nq = 3000, 262144
+    q = np.zeros((nq + 1, 4), np.float32)
+    ptr = q.ctypes.data + (-q.ctypes.data) % 16
+    best = L.Tuning()
+    h = engine.map(n, nq)
+    engine.log()
+    assert engine.lib.pm_autotune(h, 16, 32, n, L.PM_PHOTONS_PACKED, C.byref(desc(k=100)), ptr, ptr, nq, 0, C.byref(best),
+                                  None) == L.PM_OK
+    log = engine.log()
+    assert len(launched(log, "k_knn_shared<false, false>")) == 2 * 5 * 2   # each is timed the second time
+    assert all(" block 128 " in x for x in launched(log, "k_knn_group<32, true, false, true>"))
+    assert len(launched(log, "k_knn_group<32, false, false, false>")) == 2 * 5 * 3 * 2
+    engine.lib.pm_destroy(h)
+
+    b = C.c_void_p()
+    assert engine.lib.pm_batch_create(C.byref(b)) == L.PM_OK
+    photons, queries, descs = (C.c_uint32 * 2)(0, n), (C.c_uint32 * 2)(0, nq), (L.QueryDesc * 1)(desc(k=100))
+    assert engine.lib.pm_batch_autotune(b, 16, 32, photons, 1, L.PM_PHOTONS_PACKED, descs, 48, 64, queries, 80,
+                                        C.byref(best), None) == L.PM_OK
+    log = engine.log()
+    assert len(launched(log, "k_knn_shared<true, false>")) == 2 * 5 * 2
+    assert all(" block 128 " in x for x in launched(log, "k_knn_group<32, true, true, true>"))
+    assert engine.lib.pm_batch_destroy(b) == L.PM_OK
