@@ -1618,16 +1618,23 @@ static uint32_t grid_full(K kernel, int threads, int smem) {
 // lowered: a launch this small is bound by its longest warp, and a query
 // without its predecessor's radius bound costs less than waiting for it (4,095
 // queries, 1M photons, k = 100: 183 -> 58 us).
-static uint32_t grid_of(uint32_t full, uint32_t rounds, int warps_per_block, uint32_t& chunk) {
-    const uint32_t fair = rounds / (full * (uint32_t)warps_per_block);
+// The lowered chunk is rounded up where that keeps every warp to one chunk: with one
+// round less a few warps take a second chunk and the launch waits for them (65,536
+// unsorted queries, 1M photons, k = 50: warp each 699 / 549 us, four a warp 1,764 /
+// 1,272).  A small sorted launch is the exception: its queries differ more in cost
+// than in number, and shorter chunks even that out (16,384 queries: 165 us, rounded
+// up 179).
+static uint32_t grid_of(uint32_t full, uint32_t rounds, int warps_per_block, bool sorted, uint32_t& chunk) {
+    const uint32_t warps = full * (uint32_t)warps_per_block;
+    const uint32_t fair = sorted && rounds < 4u * warps ? rounds / warps : (uint32_t)(((uint64_t)rounds + warps - 1) / warps);
     if (chunk > fair) chunk = fair > 1 ? fair : 1;
     const uint32_t chunks = (rounds + chunk - 1) / chunk;
     const uint32_t need = (chunks + warps_per_block - 1) / warps_per_block;
     return full > need ? need : full;
 }
 template <class K>
-static uint32_t grid_for(K kernel, int threads, int smem, uint32_t rounds, int warps_per_block, uint32_t& chunk) {
-    return grid_of(grid_full(kernel, threads, smem), rounds, warps_per_block, chunk);
+static uint32_t grid_for(K kernel, int threads, int smem, uint32_t rounds, int warps_per_block, bool sorted, uint32_t& chunk) {
+    return grid_of(grid_full(kernel, threads, smem), rounds, warps_per_block, sorted, chunk);
 }
 
 // Whether enough queries are at hand to share walks (k_knn_shared).  Eight
@@ -1682,7 +1689,7 @@ static void launch_shared(KnnArgs a, uint32_t kmax, uint32_t nq, uint32_t* shape
         // without a bound, short ones keep a chunk in a dense blob from outlasting
         // the rest
         a.rounds_max = std::min(32u, std::max(4u, rounds / (2u * most)));
-        const uint32_t grid = grid_of(most / warps, rounds, (int)warps, a.rounds_per_chunk);
+        const uint32_t grid = grid_of(most / warps, rounds, (int)warps, true, a.rounds_per_chunk);
         kernel<<<grid, 32 * warps, a.smem_per_warp * warps, st>>>(a);
     };
     if (a.out_nbr) launch(k_knn_shared<kBatch, true>);
@@ -1703,7 +1710,7 @@ int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const 
     cudaMemsetAsync(work_counter, 0, 3 * sizeof(uint32_t), st);   // work, fix count, fix work
     if (t.layout == 0) {   // one lane per query, shared-memory heap
         const int smem = query_smem_bytes_per_warp(p.k) * t.warps_per_block;
-        const uint32_t grid = grid_for(k_knn_tree, threads, smem, (nq + 31u) / 32u, t.warps_per_block, a.rounds_per_chunk);
+        const uint32_t grid = grid_for(k_knn_tree, threads, smem, (nq + 31u) / 32u, t.warps_per_block, order != nullptr, a.rounds_per_chunk);
         k_knn_tree<<<grid, threads, smem, st>>>(a);
         *t.kernel = "k_knn_tree";
         return 1;
@@ -1727,10 +1734,10 @@ int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const 
             launch_shared<false>(a, p.k, nq, t.shared_shapes, st);
             *t.kernel = "k_knn_shared";
         } else {
-            const uint32_t grid = grid_for(k_knn_group<32, false, false, true>, threads, smem, nq, t.warps_per_block, a.rounds_per_chunk);
+            const uint32_t grid = grid_for(k_knn_group<32, false, false, true>, threads, smem, nq, t.warps_per_block, order != nullptr, a.rounds_per_chunk);
             k_knn_group<32, false, false, true><<<grid, threads, smem, st>>>(a);
         }
-        const uint32_t gfix = grid_for(k_knn_group<32, true, false, true>, threads, smem, nq, t.warps_per_block, fx.rounds_per_chunk);
+        const uint32_t gfix = grid_for(k_knn_group<32, true, false, true>, threads, smem, nq, t.warps_per_block, order != nullptr, fx.rounds_per_chunk);
         k_knn_group<32, true, false, true><<<gfix, threads, smem, st>>>(fx);
         return 2;
     }
@@ -1750,9 +1757,9 @@ int query_knn(const MapView& m, const QueryParams& p, const float4* qpos, const 
     fx.rounds_per_chunk = 1;
 #define PM_LAUNCH_GROUP(G)                                                                          \
     {                                                                                               \
-        const uint32_t grid = grid_for(k_knn_group<G, false, false, false>, threads, smem, rounds, t.warps_per_block, a.rounds_per_chunk); \
+        const uint32_t grid = grid_for(k_knn_group<G, false, false, false>, threads, smem, rounds, t.warps_per_block, order != nullptr, a.rounds_per_chunk); \
         k_knn_group<G, false, false, false><<<grid, threads, smem, st>>>(a);                                      \
-        const uint32_t gfix = grid_for(k_knn_group<G, true, false, false>, threads, smem, rounds, t.warps_per_block, fx.rounds_per_chunk); \
+        const uint32_t gfix = grid_for(k_knn_group<G, true, false, false>, threads, smem, rounds, t.warps_per_block, order != nullptr, fx.rounds_per_chunk); \
         k_knn_group<G, true, false, false><<<gfix, threads, smem, st>>>(fx);                                      \
     }
     switch (qpw) {
@@ -1800,10 +1807,10 @@ static int launch_batch(const MapView& m, const BatchQuery* bq, const BatchGeom*
         a.qsorted = t.qsorted;
         launch_shared<true>(a, kmax, nq, t.shared_shapes, st);
     } else {
-        const uint32_t grid = grid_for(k_knn_group<32, false, true, kW>, threads, smem, nq, t.warps_per_block, a.rounds_per_chunk);
+        const uint32_t grid = grid_for(k_knn_group<32, false, true, kW>, threads, smem, nq, t.warps_per_block, order != nullptr, a.rounds_per_chunk);
         k_knn_group<32, false, true, kW><<<grid, threads, smem, st>>>(a);
     }
-    const uint32_t gfix = grid_for(k_knn_group<32, true, true, kW>, threads, smem, nq, t.warps_per_block, fx.rounds_per_chunk);
+    const uint32_t gfix = grid_for(k_knn_group<32, true, true, kW>, threads, smem, nq, t.warps_per_block, order != nullptr, fx.rounds_per_chunk);
     k_knn_group<32, true, true, kW><<<gfix, threads, smem, st>>>(fx);
     return 2;
 }

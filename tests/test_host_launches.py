@@ -276,3 +276,22 @@ def test_autotuners_time_a_shared_walk_once_per_leaf_and_rounds(engine):
     assert len(launched(log, "k_knn_shared<true, false>")) == 2 * 5 * 2
     assert all(" block 128 " in x for x in launched(log, "k_knn_group<32, true, true, true>"))
     assert engine.lib.pm_batch_destroy(b) == L.PM_OK
+
+
+@pytest.mark.parametrize("nq,layout,qpw,order,blocks", [
+    # 148 SMs of 8 blocks of 4 warps: a chunk of 14 rounds keeps 65,536 queries to one for each of 4,736 warps
+    (65536, L.PM_KBUF_WIDE, 1, L.PM_ORDER_AS_GIVEN, 1171), (65536, L.PM_KBUF_WIDE, 1, L.PM_ORDER_SORTED, 1171),
+    (16384, L.PM_KBUF_WIDE, 1, L.PM_ORDER_AS_GIVEN, 1024),       # 4 rounds, 4,096 warps
+    (16384, L.PM_KBUF_WIDE, 1, L.PM_ORDER_SORTED, 1184),         # 3 rounds, 5,462 chunks
+    (4095, L.PM_KBUF_WIDE, 1, L.PM_ORDER_SORTED, 1024),          # a round each
+])
+def test_chunks_of_small_launches(engine, nq, layout, qpw, order, blocks):
+    n = 1000
+    h = engine.map(n, nq)
+    assert engine.lib.pm_set_tuning(h, 32, 4, 32, qpw, layout) == L.PM_OK
+    assert engine.build(h, n) == L.PM_OK
+    engine.log()
+    assert engine.query(h, nq, order=order) == L.PM_OK
+    (line,) = [x for x in engine.log() if "k_knn_group<32, false, false" in x and x.startswith("launch")]
+    assert f" grid {blocks} block 128 " in line
+    engine.lib.pm_destroy(h)
