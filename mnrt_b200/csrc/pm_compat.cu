@@ -32,8 +32,8 @@
 // not one per photon.  The root-to-leaf path of a query is a thread's.  With a
 // thread per query and per slot throughout the kernels ran at the pace of the
 // slots beside the blob: 300,001 photons (20 % in a caustic of sigma 0.01),
-// 307,200 queries, k = 50, R = 0.1, build included: 54.9 -> 2.9 ms; 1,500 photons
-// and 4,000 radii: 350 -> 79 us.  Latency bounds what is left (dependent node
+// 307,200 queries, k = 50, R = 0.1, build included: 54.7 -> 2.81 ms; 1,500 photons
+// and 4,000 radii: 343 -> 78 us.  Latency bounds what is left (dependent node
 // loads; a quarter of the warps' slots is taken).
 //
 // Ranges of no more than two leaves are the exception: a warp has 30 lanes too

@@ -378,9 +378,8 @@ def test_radix_sort_and_scan_through_tree_order(cuda, n):
 @pytest.mark.parametrize("chunks,pinned", [(1, True), (3, True), (1, False), (4, False), (16, True)])
 def test_build_query_host_matches_device_calls(cuda, chunks, pinned):
     """pm_build_query_host (host buffers, chunked and overlapped) gives the
-    bits of pm_build + pm_query on device buffers: a page-locked radiance
-    array written in place by the query kernel, a pageable one through a
-    device copy."""
+    bits of pm_build + pm_query on device buffers, with page-locked and
+    pageable host arrays."""
     from mnrt_b200.photon_map import PhotonMap
     ph = gen.photons(80000, seed=71, caustic_frac=0.2)
     q = gen.queries(30001, seed=72)
