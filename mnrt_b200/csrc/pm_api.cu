@@ -54,6 +54,7 @@ struct pm_map {
     DevBuf stats;           // query counters (profiling level 2)
     uint32_t shared_shapes[kSharedShapes] = {};   // QueryTuning::shared_shapes
     const char* query_kernel = "";
+    SmallSortFits fits[3];        // of the build's cluster sort, the queries' Hilbert and Morton sorts
     // backward (pm_query_backward): pair sort, per-query records, segments,
     // FP64 running sums, and the forward outputs when the kNN is recomputed
     DevBuf bvals, bvals1, bkeys0, bkeys1, bscratch, blong, qrec, seg_start, seg_end, acc;
@@ -246,6 +247,7 @@ pm_status validate_desc(pm_map* m, const pm_query_desc* d, bool exact_only, bool
 
 BuildBuffers build_buffers(pm_map* m) {
     BuildBuffers bb;
+    bb.fits = &m->fits[0];
     const size_t lane = build_block_lane(m->cap_photons);
     uint32_t* w = align32<uint32_t>(m->build_block);
     bb.keys[0] = reinterpret_cast<uint64_t*>(w); bb.keys[1] = reinterpret_cast<uint64_t*>(w + 2 * lane);
@@ -307,7 +309,7 @@ const uint32_t* sort_queries(pm_map* m, const float4* qpos, uint32_t nq, cudaStr
                              bool hilbert = true, const float4* qnrm = nullptr) {
     uint32_t* const keys[2] = {P<uint32_t>(m->qkeys0), P<uint32_t>(m->qkeys1)};
     uint32_t* const vals[2] = {P<uint32_t>(m->qvals0), P<uint32_t>(m->qvals1)};
-    return query_order(qpos, nq, P<MapHeader>(m->hdr), keys, vals, P<uint32_t>(m->qscratch), st, launches, hilbert, qnrm,
+    return query_order(qpos, nq, P<MapHeader>(m->hdr), keys, vals, P<uint32_t>(m->qscratch), &m->fits[1], st, launches, hilbert, qnrm,
                        qnrm ? P<float4>(m->qsorted) : nullptr);
 }
 
@@ -1222,7 +1224,7 @@ extern "C" pm_status pm_query_noalloc(pm_map* m, const pm_query_desc* desc, cons
         uint32_t* vals[2] = {reinterpret_cast<uint32_t*>(base + kNoallocVals0),
                              reinterpret_cast<uint32_t*>(base + kNoallocVals1)};
         order = query_order(qpos, nq, P<MapHeader>(m->hdr), keys, vals, reinterpret_cast<uint32_t*>(base + kNoallocSort),
-                            st, &nl, true);
+                            &m->fits[1], st, &nl, true);
     }
     QueryTuning t = tuning_of(m);
     t.stats = nullptr;

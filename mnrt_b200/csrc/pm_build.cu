@@ -607,9 +607,9 @@ int build_map(const float4* in_pos, const float4* in_pow, uint32_t n, int format
     const bool fuse = n > 1 && n <= kGatherInSortMax;
     bool sorted = false;
     if (n > 1 && n <= kSmallSortMax) {
-        if (n <= kSmallSortMax / 4) sorted = launch_small_sort<uint64_t, 1>(k_small_build<1>, n, st, in_pos, in_pow, n, g, keys[0], hdr);
-        else if (n <= kSmallSortMax / 2) sorted = launch_small_sort<uint64_t, 2>(k_small_build<2>, n, st, in_pos, in_pow, n, g, keys[0], hdr);
-        else sorted = launch_small_sort<uint64_t, 4>(k_small_build<4>, n, st, in_pos, in_pow, n, g, keys[0], hdr);
+        if (n <= kSmallSortMax / 4) sorted = launch_small_sort<uint64_t, 1>(k_small_build<1>, n, *bb.fits, st, in_pos, in_pow, n, g, keys[0], hdr);
+        else if (n <= kSmallSortMax / 2) sorted = launch_small_sort<uint64_t, 2>(k_small_build<2>, n, *bb.fits, st, in_pos, in_pow, n, g, keys[0], hdr);
+        else sorted = launch_small_sort<uint64_t, 4>(k_small_build<4>, n, *bb.fits, st, in_pos, in_pow, n, g, keys[0], hdr);
         if (sorted) ++nl;
     }
     if (!sorted) {

@@ -107,7 +107,22 @@ struct MapView {
     uint32_t n;             // photon count (host copy)
 };
 
+// Which sizes of a cluster sort (pm_sort_small.cuh) a handle has asked for, and
+// which of them fit; one for each kernel.
+struct SmallSortFits {
+    uint32_t size[8] = {}, count = 0;   // size << 1 | fits (a kernel has seven sizes)
+    bool find(uint32_t s, bool& fit) const {
+        for (uint32_t i = 0; i < count; ++i)
+            if (size[i] >> 1 == s) { fit = size[i] & 1u; return true; }
+        return false;
+    }
+    bool asked(uint32_t s) const { bool f; return find(s, f); }
+    bool holds(uint32_t s) const { bool f; return find(s, f) && f; }
+    void keep(uint32_t s, bool fit) { if (count < 8) size[count++] = s << 1 | (fit ? 1u : 0u); }
+};
+
 struct BuildBuffers {
+    SmallSortFits* fits;    // of k_small_build
     uint64_t* keys[2];
     uint32_t* vals[2];
     uint32_t* scratch;      // sort / scan scratch
@@ -167,10 +182,10 @@ struct QueryOutputs {
 
 // Processing order of the queries (Hilbert, or Morton); with recs also their
 // records in that order (needs the normals).  keys and vals: two buffers of nq
-// words each, scratch: sort_scratch_words(nq).
+// words each, scratch: sort_scratch_words(nq), fits: of the Hilbert and the Morton sort.
 const uint32_t* query_order(const float4* qpos, uint32_t nq, const MapHeader* hdr, uint32_t* const keys[2],
-                            uint32_t* const vals[2], uint32_t* scratch, cudaStream_t st, int* launches, bool hilbert,
-                            const float4* qnrm = nullptr, float4* recs = nullptr);
+                            uint32_t* const vals[2], uint32_t* scratch, SmallSortFits* fits, cudaStream_t st, int* launches,
+                            bool hilbert, const float4* qnrm = nullptr, float4* recs = nullptr);
 constexpr int kQueryKeyBits = 30;         // bits of the query Hilbert keys (sorted as uint32)
 constexpr int kBatchQueryMapShift = 30;   // batch query keys: (map id << 30) | 30-bit Hilbert index in the map's cell
 constexpr uint32_t kSharedShapes = 2 * (kMaxK + 1);   // by k, without and with neighbour lists

@@ -1524,17 +1524,17 @@ __global__ void __launch_bounds__(kSmallSortThreads, 1) k_small_query_sort(const
 
 template <bool kHilbert>
 static bool small_query_sort(const float4* qpos, const float4* qnrm, uint32_t nq, const MapHeader* hdr, uint32_t* order,
-                             float4* recs, cudaStream_t st) {
-    if (nq <= kSmallSortMax / 4) return launch_small_sort<uint32_t, 1>(k_small_query_sort<kHilbert, 1>, nq, st, qpos, qnrm, nq, hdr, order, recs);
-    if (nq <= kSmallSortMax / 2) return launch_small_sort<uint32_t, 2>(k_small_query_sort<kHilbert, 2>, nq, st, qpos, qnrm, nq, hdr, order, recs);
-    return launch_small_sort<uint32_t, 4>(k_small_query_sort<kHilbert, 4>, nq, st, qpos, qnrm, nq, hdr, order, recs);
+                             float4* recs, SmallSortFits& fits, cudaStream_t st) {
+    if (nq <= kSmallSortMax / 4) return launch_small_sort<uint32_t, 1>(k_small_query_sort<kHilbert, 1>, nq, fits, st, qpos, qnrm, nq, hdr, order, recs);
+    if (nq <= kSmallSortMax / 2) return launch_small_sort<uint32_t, 2>(k_small_query_sort<kHilbert, 2>, nq, fits, st, qpos, qnrm, nq, hdr, order, recs);
+    return launch_small_sort<uint32_t, 4>(k_small_query_sort<kHilbert, 4>, nq, fits, st, qpos, qnrm, nq, hdr, order, recs);
 }
 
 const uint32_t* query_order(const float4* qpos, uint32_t nq, const MapHeader* hdr, uint32_t* const keys[2],
-                            uint32_t* const vals[2], uint32_t* scratch, cudaStream_t st, int* launches, bool hilbert,
-                            const float4* qnrm, float4* recs) {
-    if (nq > 1 && nq <= kSmallSortMax && (hilbert ? small_query_sort<true>(qpos, qnrm, nq, hdr, vals[0], recs, st)
-                                                  : small_query_sort<false>(qpos, qnrm, nq, hdr, vals[0], recs, st))) {
+                            uint32_t* const vals[2], uint32_t* scratch, SmallSortFits* fits, cudaStream_t st, int* launches,
+                            bool hilbert, const float4* qnrm, float4* recs) {
+    if (nq > 1 && nq <= kSmallSortMax && (hilbert ? small_query_sort<true>(qpos, qnrm, nq, hdr, vals[0], recs, fits[0], st)
+                                                  : small_query_sort<false>(qpos, qnrm, nq, hdr, vals[0], recs, fits[1], st))) {
         ++*launches;
         return vals[0];
     }

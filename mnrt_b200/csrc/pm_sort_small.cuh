@@ -163,9 +163,11 @@ inline uint32_t small_sort_blocks(uint32_t n, int R) {
 // nothing enqueued and no error left, where that cluster does not fit (up to 16
 // blocks of 1,024 threads at once is more than a context limited to part of the
 // SMs may have) or the launch is refused: the caller then takes the sort of
-// several kernels.
+// several kernels.  Whether a size fits is asked once and kept in fits, the
+// handle's for this kernel (asked on every call: 65,536 photons and 16,384 queries
+// 240.5 us in place of 240.0, 4,095 queries 77.7 in place of 77.0).
 template <class Key, int R, class... Params, class... Args>
-inline bool launch_small_sort(void (*kernel)(Params...), uint32_t n, cudaStream_t st, Args... args) {
+inline bool launch_small_sort(void (*kernel)(Params...), uint32_t n, SmallSortFits& fits, cudaStream_t st, Args... args) {
     constexpr int smem = small_sort_smem_bytes<Key, R>();
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -178,11 +180,16 @@ inline bool launch_small_sort(void (*kernel)(Params...), uint32_t n, cudaStream_
     cfg.stream = st;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    int clusters = 0;
-    const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
-                    cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                    cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0 &&
-                    cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
+    const uint32_t size = (uint32_t)R * 32u + at[0].val.clusterDim.x;   // R at most 4, at most 16 blocks
+    bool ok = fits.holds(size);
+    if (!ok && !fits.asked(size)) {
+        int clusters = 0;
+        ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+             cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+             cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
+        fits.keep(size, ok);
+    }
+    ok = ok && cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
     if (!ok) cudaGetLastError();
     return ok;
 }

@@ -127,9 +127,9 @@ def test_small_sorts_without_room_for_a_cluster(engine, setting, value, n):
     """Maps and query sets of up to 65,536 elements take the sorts of several
     kernels where one cluster does not fit, or its launch is refused."""
     several = ["k_bounds", "k_morton", "k_digit_scatter<unsigned long", "k_query_order", "k_digit_scatter<unsigned int"]
-    h = engine.map(n, n)
     try:
         for fits in (True, False):
+            h = engine.map(n, n)
             engine.set(setting, value if not fits else {"clusters": 8, "refuse_clusters": 0}[setting])
             engine.log()
             assert engine.build(h, n) == L.PM_OK and engine.query(h, n) == L.PM_OK
@@ -137,10 +137,14 @@ def test_small_sorts_without_room_for_a_cluster(engine, setting, value, n):
             assert len(launched(log, "k_small_build")) == len(launched(log, "k_small_query_sort")) == (1 if fits else 0)
             assert [bool(launched(log, x)) for x in several] == [not fits] * len(several)
             assert launched(log, "k_knn_group")
+            assert engine.build(h, n) == L.PM_OK and engine.query(h, n) == L.PM_OK   # asked once, answered alike
+            again = engine.log()
+            assert not [x for x in again if x.startswith("clusters ")] and [x for x in log if x.startswith("clusters ")]
+            assert bool(launched(again, "k_small_build")) == bool(launched(again, "k_small_query_sort")) == fits
+            engine.lib.pm_destroy(h)
     finally:
         engine.set("clusters", 8)
         engine.set("refuse_clusters", 0)
-        engine.lib.pm_destroy(h)
 
 
 @pytest.mark.parametrize("nq,shared", [(262143, False), (262144, True)])
